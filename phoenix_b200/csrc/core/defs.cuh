@@ -91,6 +91,20 @@ PHX_HD T fmod_t(T x, T y) {
 #endif
 }
 
+// a b and a b + c with the rounding spelled out in FP32 device code: mul_1 is never contracted into an addition, fma_1
+// always rounds once.  The plasma stage uses them where its result decides something (emission cuts), so that every
+// kernel built from it (register cap, frequency slots, queue) decides alike; left to the compiler, the choice changed
+// with the code around it and moved about 7 of 3e8 samples across a cut.  FP64 and host code keep plain arithmetic.
+#if defined(__CUDA_ARCH__)
+PHX_D float mul_1(float a, float b) { return __fmul_rn(a, b); }
+PHX_D float fma_1(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+#else
+inline float mul_1(float a, float b) { return a * b; }
+inline float fma_1(float a, float b, float c) { return a * b + c; }
+#endif
+PHX_HD double mul_1(double a, double b) { return a * b; }
+PHX_HD double fma_1(double a, double b, double c) { return a * b + c; }
+
 template <class T>
 PHX_HD T sq(T x) {
   return x * x;

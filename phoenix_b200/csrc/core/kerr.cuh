@@ -185,6 +185,56 @@ PHX_HD Contra<T> contra_metric(const KerrPt<T>& p, T a) {
   return u;
 }
 
+// Geometry of a plasma sample at radius r: kerr_point_r with every rounding spelled out (mul_1, fma_1), as the emission
+// cuts depend on it.  kSig: which product of Sigma = r^2 + a^2 cos^2 is rounded before the sum (true: a^2 cos^2).
+template <class T, bool kSig>
+PHX_HD KerrPt<T> sample_point(T a, T hs, T r, T x2) {
+  T sx, cx;
+  sincos_t(x2, &sx, &cx);
+  const T s2x = mul_1(mul_1(T(2), sx), cx), c2x = (cx - sx) * (cx + sx);
+  const T d = mul_1(mul_1(T(0.5), hs), s2x);
+  KerrPt<T> p;
+  if (fabs_t(hs) <= T(1)) {
+    T sd, cd;
+    sincos_small(d, &sd, &cd);
+    p.s = fma_1(sx, cd, mul_1(cx, sd));
+    p.c = fma_1(cx, cd, -mul_1(sx, sd));
+  } else {
+    sincos_t(x2 + d, &p.s, &p.c);
+  }
+  p.r = r;
+  p.tp = fma_1(hs, c2x, T(1));
+  p.tpp = T(-2) * hs * s2x;
+  p.s2 = mul_1(p.s, p.s);
+  const T a2c = mul_1(mul_1(a, a), p.c);
+  p.sig = kSig ? fma_1(r, r, mul_1(a2c, p.c)) : fma_1(a2c, p.c, mul_1(r, r));
+  p.isig = fastm::rcp(p.sig);
+  p.q = mul_1(mul_1(T(2), r), p.isig);
+  return p;
+}
+
+// The metric of a plasma sample (cov_metric, contra_metric with the roundings spelled out; kGtt: g^tt with one rounding
+// instead of two).
+template <class T, bool kGtt>
+PHX_HD void sample_metric(const KerrPt<T>& p, T a, Cov<T>* g, Contra<T>* u) {
+  const T opq = T(1) + p.q, as2 = mul_1(-a, p.s2);
+  g->tt = p.q - T(1);
+  g->t1 = mul_1(p.q, p.r);
+  g->t3 = mul_1(as2, p.q);
+  g->x11 = mul_1(mul_1(opq, p.r), p.r);
+  g->x13 = mul_1(mul_1(as2, opq), p.r);
+  g->x22 = mul_1(mul_1(p.sig, p.tp), p.tp);
+  g->x33 = mul_1(p.s2, fma_1(mul_1(mul_1(a, a), p.s2), opq, p.sig));
+  const T ir = fastm::rcp(p.r), tp2 = mul_1(p.tp, p.tp);
+  const T iprod = mul_1(p.isig, fastm::rcp(mul_1(tp2, p.s2)));
+  u->tt = kGtt ? -fma_1(mul_1(T(2), p.r), p.isig, T(1)) : -opq;
+  u->t1 = mul_1(T(2), p.isig);
+  u->x11 = mul_1(mul_1(mul_1(p.isig, fma_1(p.r - T(2), p.r, mul_1(a, a))), ir), ir);
+  u->x13 = mul_1(mul_1(a, p.isig), ir);
+  u->x22 = mul_1(iprod, p.s2);
+  u->x33 = mul_1(iprod, tp2);
+}
+
 // Inner product of a lowered vector with a vector.
 template <class T>
 PHX_HD T dot4(const T Ud[4], const T V[4]) {

@@ -128,6 +128,10 @@ struct Ray {
   static constexpr bool kWP = !kLate;
   static constexpr int kNS = kWP ? 8 : 12;
 
+  // the one-slot mixed kernels round the sample's Sigma the other way than the rest (sample_point) and leave B^2 to the
+  // compiler, as they always have: a sample on an emission cut turns on the last bit
+  static constexpr bool kSig = !(kMixed && NF == 1);
+
   GeoState<G, kNS> geo;
   R kappa[2];   // Walker-Penrose constant of (k, F1) (kWP)
   G px[4], pk[4], pF[4], pdl;  // FP64 (kLate): the pending sample's point and the length of the step to it
@@ -140,7 +144,8 @@ struct Ray {
   G idxc[3];    // its inverse cell sizes (FP32 and mixed step-size cap)
   // transfer records (4x4 operator, Stokes sums, optical depths) per frequency slot: the kernels of 4 slots and the
   // mixed and FP64 kernels of 1 keep them in the block's dynamic shared memory (kSmemPerThread bytes per thread), the
-  // FP32 one-slot and all 32-slot kernels in registers.  Measured on B200: mixed 3-frequency renders 14% faster,
+  // FP32 one-slot kernel in registers, the 32-slot kernels in the thread's local memory (3 to 6 KB a thread, of which a
+  // pass touches nfreqs records; interleaved by lane, so a warp's access is whole lines).  Measured on B200: mixed 3-frequency renders 14% faster,
   // FP64 3-5%, FP32 3-frequency 3-6% (no spills at 128 registers); FP32 with one slot 3% slower, so it keeps
   // registers.
   // Host builds (g++: tools and the host tests of this code) have no shared memory and keep the records in the object.
@@ -177,7 +182,7 @@ struct Ray {
     geo_init<G, kComp>(geo, st.ph, st.F1);
     kappa[0] = R(st.kappa[0]);
     kappa[1] = R(st.kappa[1]);
-#pragma unroll
+#pragma unroll 1
     for (int f = 0; f < NF; f++) acc_reset<R, kMixed>(acc, f);
     pvalid = false;
     terminate = false;
@@ -338,11 +343,12 @@ struct Ray {
     const R x2w = R(xg[2]);
     const R rx = R(r);
     R k[4] = {R(kg[0]), R(kg[1]), R(kg[2]), R(kg[3])};
-    const KerrPt<R> p = kerr_point_r(s.a, s.hs, rx, x2w);
-    const Cov<R> g = cov_metric(p, s.a);
-    const Contra<R> u = contra_metric(p, s.a);
+    const KerrPt<R> p = sample_point<R, kSig>(s.a, s.hs, rx, x2w);
+    Cov<R> g;
+    Contra<R> u;
+    sample_metric<R, !kMixed || (NF > 4)>(p, s.a, &g, &u);
     Fluid<R> fl;
-    if (!derive_fluid(rc.pv, s.gam, rx, g, u, q, &fl)) return;
+    if (!derive_fluid<R, kSig>(rc.pv, s.gam, rx, g, u, q, &fl)) return;
     if (!(r < rc.template steps_in<G>().rt_outer)) return;
     // k, U and B lowered once: every invariant below is then a 4-term inner product
     R kd[4], Ud[4], Bd[4];
@@ -395,9 +401,14 @@ struct Ray {
     const R ratio = -kU;  // nu_plasma / nu_camera
     const SynchroSample<R> ss = synchro_sample(fl.theta_e, fl.n_e, fl.Bmag, sth, cth);
     const R hlr = R(hl);
-#pragma unroll
-    for (int f = 0; f < NF; f++) {
-      if (f >= rc.nfreqs) break;
+    const int nf = NF == 1 ? 1 : rc.nfreqs;
+    // Rolled: the stage is bound by instruction issue and fetch, and one copy of the coefficients and the operator (about
+    // 400 instructions) stays in the instruction cache where 4 or 32 copies stream through it every pass; the records are
+    // indexed by f in shared or local memory.  Measured against the unrolled loop: 129 x 96, 8 frequencies, FP32 54.1 ->
+    // 39.7 ms (the 32-slot kernel spilled 5 KB a thread), 333 x 217, 3 frequencies, mixed 83.3 -> 78.8 ms, 1024^2, 3
+    // frequencies, FP32 462 -> 442 ms with the host's share.
+#pragma unroll 1
+    for (int f = 0; f < nf; f++) {
       const R nu = rc.freq[f] * ratio;
       const Coeffs<R> cf = synchro_coeffs(ss, nu, rc.jscale[f]);
       R K[4][4], jv[4], E[4][4], Sg[4];
@@ -435,9 +446,9 @@ struct Ray {
 
   // FreqOut records (I, Q, U, V, tau, tauF as doubles) of this pixel; zeros when no plasma segment was crossed.
   PHX_HD void write(double* out, int nfreqs) {
-#pragma unroll
-    for (int f = 0; f < NF; f++) {
-      if (f >= nfreqs) break;
+    const int nf = NF == 1 ? 1 : nfreqs;
+#pragma unroll 1
+    for (int f = 0; f < nf; f++) {
       double* o = out + ((size_t)pix * nfreqs + f) * 6;
       const bool any = nplasma > 0;
       using W = AccWords<kMixed>;

@@ -200,13 +200,13 @@ PHX_HD void cell_weights(const SnapView<R, PT>& s, int leaf, const R x[4], int c
     const R lb = ldg(s.lb + 3 * leaf + d), dx = ldg(s.dxc + 3 * leaf + d);
     // FP32: one reciprocal per axis (rounding-level difference; the interpolant is continuous across cells)
     const R idx = sizeof(R) == 4 ? fastm::rcp(dx) : R(0);
-    const R u = sizeof(R) == 4 ? (x[1 + d] - lb) * idx : (x[1 + d] - lb) / dx;
+    const R u = sizeof(R) == 4 ? mul_1(x[1 + d] - lb, idx) : (x[1 + d] - lb) / dx;
     c[d] = (int)u;
     if (c[d] >= s.nx[d]) c[d] = s.nx[d] - 1;
     if (c[d] < 0) c[d] = 0;  // unreachable for finite points of the leaf; keeps every gather inside the block
     const int ix = kFloorBy1000 ? (int)(u + R(1000)) - 1000 : (int)floor_t(u);
-    const R off = x[1 + d] - (R(ix) * dx + lb);
-    del[d] = (ix < 0) ? R(0) : (ix > s.nx[d] - 2) ? R(1) : (sizeof(R) == 4 ? off * idx : off / dx);
+    const R off = x[1 + d] - fma_1(R(ix), dx, lb);
+    del[d] = (ix < 0) ? R(0) : (ix > s.nx[d] - 2) ? R(1) : (sizeof(R) == 4 ? mul_1(off, idx) : off / dx);
   }
 }
 
@@ -221,7 +221,7 @@ PHX_HD void gather_prims(const PT* prim, int cells, const int nx[3], int leaf, c
   const R b1 = R(1) - del[0], b2 = R(1) - del[1], b3 = R(1) - del[2];
   const int ci[4] = {c[0], c[0], cip, cip};
   const int cj[4] = {c[1], cjp, c[1], cjp};
-  const R wq[4] = {b1 * b2, b1 * del[1], del[0] * b2, del[0] * del[1]};
+  const R wq[4] = {mul_1(b1, b2), mul_1(b1, del[1]), mul_1(del[0], b2), mul_1(del[0], del[1])};
   const PT* base = prim + (size_t)leaf * cells * kNPrim;
 #pragma unroll
   for (int a = 0; a < kNPrim; a++) q[a] = R(0);
@@ -251,9 +251,9 @@ PHX_HD void gather_prims(const PT* prim, int cells, const int nx[3], int leaf, c
 #else
       for (int a = 0; a < kNPrim; a++) v[a] = R(p[a]);
 #endif
-      const R w = wq[n] * wz;
+      const R w = mul_1(wq[n], wz);
 #pragma unroll
-      for (int a = 0; a < kNPrim; a++) q[a] += v[a] * w;
+      for (int a = 0; a < kNPrim; a++) q[a] = fma_1(v[a], w, q[a]);
     }
   }
 }
@@ -268,42 +268,58 @@ PHX_HD void interp_prims(const SnapView<R, PT>& s, int leaf, const R x[4], R q[k
 }
 
 // Fluid 4-velocity, magnetic 4-vector, |B| [G], n_e and Theta_e from the interpolated primitives; returns whether
-// the point emits (sampler.hpp:305-376).  g / u: metric at x.
-template <class R>
+// the point emits (sampler.hpp:305-376).  g / u: metric at x.  kSpelled: B^2 with its roundings spelled out.
+template <class R, bool kSpelled>
 PHX_HD bool derive_fluid(const PlasmaView<R>& pv, R gam, R r, const Cov<R>& g, const Contra<R>& u, const R q[kNPrim],
                          Fluid<R>* fl) {
   const R smalll = R(1e-6);
   const R rho = q[kRho], uu = q[kUU];
-  fl->n_e = rho * pv.Ne + smalll;
+  fl->n_e = fma_1(rho, pv.Ne, smalll);
   // lapse alpha = 1 / sqrt(-g^tt), shift^1 = alpha^2 g^t1; the divisions are folded into reciprocals
   const R ialpha = fastm::sqrt(-u.tt);
   const R alpha = fastm::rcp(ialpha);  // FP32: hardware reciprocals and quotients here (2 ulp); FP64: exact
-  const R shift1 = u.t1 * alpha * alpha;
+  const R shift1 = mul_1(mul_1(u.t1, alpha), alpha);
   const R gv1 = q[kU1], gv2 = q[kU2], gv3 = q[kU3];
-  const R gvv = g.x11 * gv1 * gv1 + R(2) * g.x13 * gv1 * gv3 + g.x22 * gv2 * gv2 + g.x33 * gv3 * gv3;
+  const R x13gv1 = mul_1(mul_1(R(2), g.x13), gv1);
+  const R gvv = fma_1(mul_1(g.x33, gv3), gv3,
+                      fma_1(mul_1(g.x22, gv2), gv2, fma_1(mul_1(g.x11, gv1), gv1, mul_1(x13gv1, gv3))));
   const R lfac = fastm::sqrt(gvv + R(1));
   const R ilfac = fastm::rcp(lfac);
-  const R V1 = gv1 * ilfac, V2 = gv2 * ilfac, V3 = gv3 * ilfac;
-  const R ut = lfac * ialpha;
+  const R V1 = mul_1(gv1, ilfac), V2 = mul_1(gv2, ilfac), V3 = mul_1(gv3, ilfac);
+  const R ut = mul_1(lfac, ialpha);
   fl->U[0] = ut;
-  fl->U[1] = V1 * lfac - shift1 * ut;
-  fl->U[2] = V2 * lfac;
-  fl->U[3] = V3 * lfac;
+  fl->U[1] = fma_1(V1, lfac, -mul_1(shift1, ut));
+  fl->U[2] = mul_1(V2, lfac);
+  fl->U[3] = mul_1(V3, lfac);
   const R Bp1 = q[kB1], Bp2 = q[kB2], Bp3 = q[kB3];
   // B^t = lfac (gamma_ij Bp^i V^j) / alpha
-  const R BV = Bp1 * (g.x11 * V1 + g.x13 * V3) + Bp2 * (g.x22 * V2) + Bp3 * (g.x13 * V1 + g.x33 * V3);
-  fl->B[0] = lfac * BV * ialpha;
-  fl->B[1] = (Bp1 + alpha * fl->B[0] * fl->U[1]) * ilfac;
-  fl->B[2] = (Bp2 + alpha * fl->B[0] * fl->U[2]) * ilfac;
-  fl->B[3] = (Bp3 + alpha * fl->B[0] * fl->U[3]) * ilfac;
-  const R Bsq = fabs_t(dot(g, fl->B, fl->B)) + smalll;
+  const R BV = fma_1(Bp3, fma_1(g.x13, V1, mul_1(g.x33, V3)),
+                     fma_1(Bp1, fma_1(g.x11, V1, mul_1(g.x13, V3)), mul_1(Bp2, mul_1(g.x22, V2))));
+  fl->B[0] = mul_1(mul_1(lfac, BV), ialpha);
+  const R aB0 = mul_1(alpha, fl->B[0]);
+  fl->B[1] = mul_1(fma_1(aB0, fl->U[1], Bp1), ilfac);
+  fl->B[2] = mul_1(fma_1(aB0, fl->U[2], Bp2), ilfac);
+  fl->B[3] = mul_1(fma_1(aB0, fl->U[3], Bp3), ilfac);
+  R bb2;
+  if constexpr (kSpelled) {
+    const R B0 = fl->B[0], B1 = fl->B[1], B2 = fl->B[2], B3 = fl->B[3];
+    bb2 = fma_1(mul_1(g.tt, B0), B0, mul_1(g.t1, R(2) * mul_1(B0, B1)));
+    bb2 = fma_1(g.t3, R(2) * mul_1(B0, B3), bb2);
+    bb2 = fma_1(mul_1(g.x11, B1), B1, bb2);
+    bb2 = fma_1(g.x13, R(2) * mul_1(B1, B3), bb2);
+    bb2 = fma_1(mul_1(g.x22, B2), B2, bb2);
+    bb2 = fma_1(mul_1(g.x33, B3), B3, bb2);
+  } else {
+    bb2 = dot(g, fl->B, fl->B);
+  }
+  const R Bsq = fabs_t(bb2) + smalll;
   fl->Bmag = fastm::sqrt(Bsq) * pv.Bu;
   const R beta = fastm::div(uu * (gam - R(1)), R(0.5) * (Bsq + smalll));
   const R bb = beta * pv.ibc;
-  const R b2 = bb * bb;
+  const R b2 = mul_1(bb, bb);
   const R ib2 = fastm::rcp(R(1) + b2);
-  const R trat = (pv.rhigh * b2 + pv.rlow) * ib2;
-  const R te_unit = fastm::div(R(1.0 / 3.0 * (cgs::m_proton / cgs::m_electron)), trat + R(1));
+  const R trat1 = fma_1(fma_1(pv.rhigh, b2, pv.rlow), ib2, R(1));  // T_p / T_e + 1
+  const R te_unit = fastm::div(R(1.0 / 3.0 * (cgs::m_proton / cgs::m_electron)), trat1);
   fl->theta_e = fastm::div(uu, rho) * te_unit;
   if ((fastm::div(Bsq, rho + R(1e-20)) > pv.sigma_cut) || r > pv.rt_outer || fl->theta_e > pv.thetae_max ||
       fl->theta_e < pv.thetae_min) {

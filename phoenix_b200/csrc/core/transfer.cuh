@@ -127,7 +127,7 @@ struct AccWords {
                        kN = kTau + 3;
 };
 
-// Records in the thread's registers (FP64 and the 32-slot kernels).
+// Records in the thread's registers (one slot) or, indexed by the frequency, its local memory (32 slots).
 template <class R, bool kKahan, int NF>
 struct AccRegs {
   static constexpr size_t kSmemPerThread = 0;
