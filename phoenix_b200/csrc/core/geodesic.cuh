@@ -155,9 +155,10 @@ PHX_HD void rk4_step(R a, R hs, GeoState<R, NS>& g, R dt) {
         // theta - theta0 = d2 + (h/2)(sin 2x2 - sin 2x2_0): |.| <= (1 + |h|) kShiftMax <= 0.0375
         R sdt, cdt;
         sincos_tiny(d2 + R(0.5) * hs * (s2x - s2x0), &sdt, &cdt);
-        const KerrPt<R> p = kerr_point_theta<R, true>(a, hs, e0 * exp_small<R, 7>(d1), s2x, c2x,
-                                                      st0 * cdt + ct0 * sdt, ct0 * cdt - st0 * sdt);
-        geodesic_accel_at<R, kF, true>(a, p, y + 4, y + 8, d + 4, d + 8);
+        static_assert(!kF, "the shifted stages transport no polarization vector");
+        const KsPt<R> p = {e0 * exp_small<R, 7>(d1), st0 * cdt + ct0 * sdt, ct0 * cdt - st0 * sdt,
+                           R(1) + hs * c2x, R(-2) * hs * s2x};
+        geodesic_accel_ks(a, p, y + 4, d + 4);
       } else {
         StagePoint<R> sp;
         sp.a = a;
