@@ -115,48 +115,19 @@ struct RayCounters {
   uint32_t steps, nplasma, bad, scans, fp64_steps, fp64_ops;
 };
 
-template <Mode M, class PT, int NF>
-struct Ray {
+// The types of a mode's ray.
+template <Mode M, class PT>
+struct RayTypes {
   using Pol = Policy<M>;
   using R = typename Pol::R;
   using G = typename Pol::G;
   static constexpr bool kComp = Pol::kComp, kMixed = Pol::kMixed, kShift = Pol::kShift;
-  static constexpr bool kLate = M == Mode::kFP64;  // the reference's one-pass-late sample order (see advance())
+  static constexpr bool kLate = M == Mode::kFP64;  // the reference's one-pass-late sample order (see GeoRay::march)
   // FP32 and mixed: the polarization direction at a sample comes from the Walker-Penrose constant taken at the camera
   // (exact for parallel transport), so the geodesic state is (x, k) only; FP64 transports F1 with the state as the
   // reference does, and follows it bit for bit
   static constexpr bool kWP = !kLate;
   static constexpr int kNS = kWP ? 8 : 12;
-
-  // the one-slot mixed kernels round the sample's Sigma the other way than the rest (sample_point) and leave B^2 to the
-  // compiler, as they always have: a sample on an emission cut turns on the last bit
-  static constexpr bool kSig = !(kMixed && NF == 1);
-
-  GeoState<G, kNS> geo;
-  R kappa[2];   // Walker-Penrose constant of (k, F1) (kWP)
-  G px[4], pk[4], pF[4], pdl;  // FP64 (kLate): the pending sample's point and the length of the step to it
-  bool pvalid, terminate;
-  int steps, turns, bsign, nplasma, bad;
-  G thdot_prev, dl_prev;
-  G pr;         // radius of the pending sample (exp of px[1], from the step that made it)
-  int32_t pix;
-  int leaf;     // leaf of the last step-size lookup (-1: none), tested before the leaf map
-  G idxc[3];    // its inverse cell sizes (FP32 and mixed step-size cap)
-  // transfer records (4x4 operator, Stokes sums, optical depths) per frequency slot: the kernels of 4 slots and the
-  // mixed and FP64 kernels of 1 keep them in the block's dynamic shared memory (kSmemPerThread bytes per thread), the
-  // FP32 one-slot kernel in registers, the 32-slot kernels in the thread's local memory (3 to 6 KB a thread, of which a
-  // pass touches nfreqs records; interleaved by lane, so a warp's access is whole lines).  Measured on B200: mixed 3-frequency renders 14% faster,
-  // FP64 3-5%, FP32 3-frequency 3-6% (no spills at 128 registers); FP32 with one slot 3% slower, so it keeps
-  // registers.
-  // Host builds (g++: tools and the host tests of this code) have no shared memory and keep the records in the object.
-#if defined(__CUDACC__)
-  static constexpr bool kAccShared = (kMixed || M == Mode::kFP64 || NF > 1) && NF <= 4;
-#else
-  static constexpr bool kAccShared = false;
-#endif
-  using AccStore = std::conditional_t<kAccShared, AccShared<R, kMixed, NF>, AccRegs<R, kMixed, NF>>;
-  static constexpr size_t kSmemPerThread = AccStore::kSmemPerThread;
-  AccStore acc;
 
   // The snapshot in the geodesic's precision: the plasma-stage view itself (FP32, FP64) or the FP64 view sd (mixed).
   // Both live in kernel parameter space or in the item table, so no copy is made for the out-of-line callees that
@@ -168,25 +139,32 @@ struct Ray {
       return sd;
     }
   }
+};
 
-  PHX_HD void init(const SnapView<R, PT>& s, const SnapView<double, PT>& sd, const RenderConsts<R>& rc,
-                   int32_t pixel) {
-    const SnapView<G, PT>& sg = geo_view(s, sd);
-    init_from(ray_start<G>(rc, sg.a, sg.hs, pixel), pixel);
-  }
+// The geodesic of a ray: state, liveness, leaf cache, step size.
+template <Mode M, class PT>
+struct GeoRay : RayTypes<M, PT> {
+  using T = RayTypes<M, PT>;
+  using R = typename T::R;
+  using G = typename T::G;
+  using T::kComp, T::kLate, T::kMixed, T::kNS, T::kShift, T::kWP;
 
-  // Starts the ray from its camera set-up (ray_start), computed here or beforehand by the ray-setup kernel: the same
-  // out-of-line function either way, so the ray is bit-identical.
-  PHX_HD void init_from(const RayStart& st, int32_t pixel) {
+  GeoState<G, kNS> geo;
+  G px[4], pk[4], pF[4], pdl;  // FP64 (kLate): the pending sample's point and the length of the step to it
+  bool pvalid, terminate;
+  int steps, turns, bsign;
+  G thdot_prev, dl_prev;
+  G pr;         // radius of the pending sample (exp of px[1], from the step that made it)
+  int32_t pix;
+  int leaf;     // leaf of the last step-size lookup (-1: none), tested before the leaf map
+  G idxc[3];    // its inverse cell sizes (FP32 and mixed step-size cap)
+
+  PHX_HD void start(const RayStart& st, int32_t pixel) {
     pix = pixel;
     geo_init<G, kComp>(geo, st.ph, st.F1);
-    kappa[0] = R(st.kappa[0]);
-    kappa[1] = R(st.kappa[1]);
-#pragma unroll 1
-    for (int f = 0; f < NF; f++) acc_reset<R, kMixed>(acc, f);
     pvalid = false;
     terminate = false;
-    steps = turns = nplasma = bad = 0;
+    steps = turns = 0;
     bsign = st.bsign;
     thdot_prev = dl_prev = G(0);
     pr = G(0);
@@ -221,9 +199,11 @@ struct Ray {
   // lengths are the same (points 1.. of the live path inside rt_outer, each with the length of the step that led to
   // it), no copy of the previous point's state is carried (fewer registers), and the leaf found differs only for
   // points within the sampler's 1e-9 nudge of a block face.
-  PHX_HD bool advance(const SnapView<R, PT>& s, const SnapView<double, PT>& sd, const RenderConsts<R>& rc,
-                      RayCounters& ctr) {
-    const SnapView<G, PT>& sg = geo_view(s, sd);
+  //
+  // sample(x, k, F, r, hl, right) takes each sample as it comes: the plasma stage itself (Ray), or a store for another
+  // warp's plasma stage (the pipelined kernel).  Nothing of the geodesic depends on it.
+  template <class Sink>
+  PHX_HD bool march(const SnapView<G, PT>& sg, const RenderConsts<R>& rc, RayCounters& ctr, Sink&& sample) {
     const StepConsts<G>& sc = rc.template steps_in<G>();
     G cx[4], ck[4], cF[4];
 #pragma unroll
@@ -252,7 +232,7 @@ struct Ray {
         L = lookup(sg, xw, ctr);
         if (need_leaf) right = (r < G(1) || outside_domain(sg, xw)) ? -1 : L;  // wrapping keeps x1: exp(xw[1]) = r
       }
-      if (pend_plasma) process_sample(s, sg, rc, px, pk, pF, pr, pdl, right, ctr);
+      if (pend_plasma) sample(px, pk, pF, pr, pdl, right);
 #pragma unroll
       for (int i = 0; i < 4; i++) {
         px[i] = cx[i];
@@ -271,7 +251,7 @@ struct Ray {
         L = lookup(sg, xw, ctr);
         if (steps >= 1) {
           const int right = (r < G(1) || outside_domain(sg, xw)) ? -1 : L;  // wrapping keeps x1: exp(xw[1]) = r
-          process_sample(s, sg, rc, cx, ck, cF, r, dl_prev, right, ctr);
+          sample(cx, ck, cF, r, dl_prev, right);
         }
       }
     }
@@ -301,12 +281,38 @@ struct Ray {
     steps++;
     return true;
   }
+};
+
+// The plasma stage of a ray: its Walker-Penrose constant and its transfer records (AccStore).  It takes every kStride-th
+// frequency from `first` on (all of them: 1, 0), and keeps a record for each of those it takes.
+template <Mode M, class PT, int NF, class AccStore, int kStride = 1>
+struct PlasmaRay : RayTypes<M, PT> {
+  using T = RayTypes<M, PT>;
+  using R = typename T::R;
+  using G = typename T::G;
+  using T::kComp, T::kMixed, T::kWP;
+  // the one-slot mixed kernels round the sample's Sigma the other way than the rest (sample_point) and leave B^2 to the
+  // compiler, as they always have: a sample on an emission cut turns on the last bit
+  static constexpr bool kSig = !(kMixed && NF == 1);
+
+  R kappa[2];  // Walker-Penrose constant of (k, F1) (kWP)
+  int nplasma, bad;
+  AccStore acc;
+
+  PHX_HD void start(const double kap[2]) {
+    kappa[0] = R(kap[0]);
+    kappa[1] = R(kap[1]);
+#pragma unroll 1
+    for (int e = 0; e < (NF + kStride - 1) / kStride; e++) acc_reset<R, kMixed>(acc, e);
+    nplasma = bad = 0;
+  }
 
   // The plasma stage of the sample at point (x0, k0, F0) of radius r, reached by a step of length hl (the reference's
   // process_sample, core/render/pixel.hpp:52-123).  The point comes in the geodesic's precision G; the fluid,
   // coefficients and transfer operator run in R.
   PHX_HD void process_sample(const SnapView<R, PT>& s, const SnapView<G, PT>& sg, const RenderConsts<R>& rc,
-                             const G x0[4], const G k0[4], const G F0[4], G r, G hl, int right, RayCounters& ctr) {
+                             const G x0[4], const G k0[4], const G F0[4], G r, G hl, int right, RayCounters& ctr,
+                             int first = 0) {
     // null-condition renormalisation of the sample's wave vector, in the geodesic's precision (reference:
     // geodesic.hpp:297-306, applied when |k.k| > 1e-6 and r > 2)
     G kg[4] = {k0[0], k0[1], k0[2], k0[3]};
@@ -408,7 +414,7 @@ struct Ray {
     // 39.7 ms (the 32-slot kernel spilled 5 KB a thread), 333 x 217, 3 frequencies, mixed 83.3 -> 78.8 ms, 1024^2, 3
     // frequencies, FP32 462 -> 442 ms with the host's share.
 #pragma unroll 1
-    for (int f = 0; f < nf; f++) {
+    for (int f = first, e = 0; f < nf; f += kStride, e++) {
       const R nu = rc.freq[f] * ratio;
       const Coeffs<R> cf = synchro_coeffs(ss, nu, rc.jscale[f]);
       R K[4][4], jv[4], E[4][4], Sg[4];
@@ -439,27 +445,80 @@ struct Ray {
         bad++;
         continue;
       }
-      acc_add<R, kMixed>(acc, f, E, Sg, cf.aI * h, fabs_t(cf.rV * h));
+      acc_add<R, kMixed>(acc, e, E, Sg, cf.aI * h, fabs_t(cf.rV * h));
     }
     nplasma++;
   }
 
   // FreqOut records (I, Q, U, V, tau, tauF as doubles) of this pixel; zeros when no plasma segment was crossed.
-  PHX_HD void write(double* out, int nfreqs) {
+  PHX_HD void write(double* out, int32_t pix, int nfreqs, int first = 0) {
     const int nf = NF == 1 ? 1 : nfreqs;
 #pragma unroll 1
-    for (int f = 0; f < nf; f++) {
+    for (int f = first, e = 0; f < nf; f += kStride, e++) {
       double* o = out + ((size_t)pix * nfreqs + f) * 6;
       const bool any = nplasma > 0;
       using W = AccWords<kMixed>;
-      o[0] = any ? (double)acc.at(f, W::kS) : 0.0;
-      o[1] = any ? (double)acc.at(f, W::kS + 1) : 0.0;
-      o[2] = any ? (double)acc.at(f, W::kS + 2) : 0.0;
-      o[3] = any ? (double)acc.at(f, W::kS + 3) : 0.0;
-      o[4] = any ? (double)acc.at(f, W::kTau) : 0.0;
-      o[5] = any ? (double)acc.at(f, W::kTauF) : 0.0;
+      o[0] = any ? (double)acc.at(e, W::kS) : 0.0;
+      o[1] = any ? (double)acc.at(e, W::kS + 1) : 0.0;
+      o[2] = any ? (double)acc.at(e, W::kS + 2) : 0.0;
+      o[3] = any ? (double)acc.at(e, W::kS + 3) : 0.0;
+      o[4] = any ? (double)acc.at(e, W::kTau) : 0.0;
+      o[5] = any ? (double)acc.at(e, W::kTauF) : 0.0;
     }
   }
+};
+
+// Where the transfer records of the plain and the queue kernel live.
+template <Mode M, class PT, int NF>
+struct RayStore {
+  using T = RayTypes<M, PT>;
+  using R = typename T::R;
+  // transfer records (4x4 operator, Stokes sums, optical depths) per frequency slot: the kernels of 4 slots and the
+  // mixed and FP64 kernels of 1 keep them in the block's dynamic shared memory (kSmemPerThread bytes per thread), the
+  // FP32 one-slot kernel in registers, the 32-slot kernels in the thread's local memory (3 to 6 KB a thread, of which a
+  // pass touches nfreqs records; interleaved by lane, so a warp's access is whole lines).  Measured on B200: mixed 3-frequency renders 14% faster,
+  // FP64 3-5%, FP32 3-frequency 3-6% (no spills at 128 registers); FP32 with one slot 3% slower, so it keeps
+  // registers.
+  // Host builds (g++: tools and the host tests of this code) have no shared memory and keep the records in the object.
+#if defined(__CUDACC__)
+  static constexpr bool kAccShared = (T::kMixed || M == Mode::kFP64 || NF > 1) && NF <= 4;
+#else
+  static constexpr bool kAccShared = false;
+#endif
+  using AccStore = std::conditional_t<kAccShared, AccShared<R, T::kMixed, NF>, AccRegs<R, T::kMixed, NF>>;
+};
+
+// One ray, marched and sampled by one lane.
+template <Mode M, class PT, int NF>
+struct Ray : GeoRay<M, PT>, PlasmaRay<M, PT, NF, typename RayStore<M, PT, NF>::AccStore> {
+  using Geo = GeoRay<M, PT>;
+  using Plasma = PlasmaRay<M, PT, NF, typename RayStore<M, PT, NF>::AccStore>;
+  using R = typename Geo::R;
+  using G = typename Geo::G;
+  static constexpr size_t kSmemPerThread = RayStore<M, PT, NF>::AccStore::kSmemPerThread;
+
+  PHX_HD void init(const SnapView<R, PT>& s, const SnapView<double, PT>& sd, const RenderConsts<R>& rc,
+                   int32_t pixel) {
+    const SnapView<G, PT>& sg = Geo::geo_view(s, sd);
+    init_from(ray_start<G>(rc, sg.a, sg.hs, pixel), pixel);
+  }
+
+  // Starts the ray from its camera set-up (ray_start), computed here or beforehand by the ray-setup kernel: the same
+  // out-of-line function either way, so the ray is bit-identical.
+  PHX_HD void init_from(const RayStart& st, int32_t pixel) {
+    Geo::start(st, pixel);
+    Plasma::start(st.kappa);
+  }
+
+  PHX_HD bool advance(const SnapView<R, PT>& s, const SnapView<double, PT>& sd, const RenderConsts<R>& rc,
+                      RayCounters& ctr) {
+    const SnapView<G, PT>& sg = Geo::geo_view(s, sd);
+    return Geo::march(sg, rc, ctr, [&](const G* x, const G* k, const G* F, G r, G hl, int right) {
+      Plasma::process_sample(s, sg, rc, x, k, F, r, hl, right, ctr);
+    });
+  }
+
+  PHX_HD void write(double* out, int nfreqs) { Plasma::write(out, Geo::pix, nfreqs); }
 };
 
 }  // namespace phx

@@ -43,6 +43,7 @@ struct MarchArgs {
   unsigned long long* counters;
   int32_t period;
   int32_t refill_lanes;  // finished lanes at which a warp refills before its period ends (checked every 64 passes)
+  bool default_schedule;  // the caller named no refill policy: the launch may take the pipelined kernel
 };
 
 __device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long v) {

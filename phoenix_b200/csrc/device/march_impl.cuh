@@ -2,6 +2,7 @@
 #pragma once
 
 #include "march.cuh"
+#include "march_pipe.cuh"
 
 namespace phx {
 
@@ -43,6 +44,58 @@ cudaError_t launch_mb(const MarchArgs<typename Policy<M>::R, PT>& args, int sms,
   return cudaGetLastError();
 }
 
+// The pipelined kernel (march_pipe.cuh) takes the launches of few rays per SM.  Its blocks hold one ray per lane of their
+// geodesic warp only, so 168 registers leave room for 192 rays an SM (128: 256) against the plain kernel's 512: it wins
+// while a launch is as long as its longest rays, and loses once the rays fill the chip several times over.  ms of one
+// image at 20 / 75 deg, pipelined against plain (96^3-base snapshot; the same bits for FP64):
+//   FP32, 1 frequency:   64^2 10.5 / 10.1 against 16.2 / 16.0;  128^2 15.1 / 11.7 : 21.5 / 16.3;  200^2 17.8 / 14.2 : 23.9 / 20.6;
+//     256^2 (443 rays an SM) 20.3 / 20.8 : 26.8 / 30.3;  320^2 (692) 29.5 / 25.6, 128 registers 27.4 / 24.2 : 29.2 / 27.0;
+//     400^2 (1081) 128 registers 41.1 / 35.9 : 42.8 / 32.8;  512^2 65.6 / 56.4 : 48.4 / 42.3
+//   FP32, 3 frequencies: 128^2 18.4 / 17.5 : 22.4 / 20.0;  256^2 35.6 / 33.2, 128 registers 33.9 / 31.7 : 31.6 / 37.6;
+//     400^2 79.0 / 72.8 : 51.6 / 40.7
+//   FP32, 8 frequencies: 64^2 13.2 / 12.3 : 29.1 / 24.7;  128^2 18.2 / 16.4 : 27.1 / 27.8;  200^2 (270) 34.7 / 32.0 : 39.7 / 35.2
+//   mixed, 1 frequency:  64^2 14.8 / 15.5 : 24.9 / 25.2;  256^2 30.9 / 32.5 : 41.3 / 47.7;  320^2 128 registers 40.7 / 34.5 :
+//     45.7 / 42.4;  400^2 61.4 / 52.4 : 66.8 / 48.8;  3 frequencies, 333 x 217 (488) 54.7 / 49.1 : 60.5 / 62.7
+//   FP64, 1 frequency:   64^2 30.2 / 30.8 : 45.9 / 45.9;  200^2 (270) 69.0 / 55.7 : 79.8 / 68.2;  256^2 95.9 / 81.7 : 82.6 / 93.5
+template <Mode M, int NF>
+constexpr long long pipe_rays_per_sm() {
+  return M == Mode::kFP64 || NF > 4 ? 300 : NF > 1 ? 500 : 700;
+}
+constexpr int kPipeWideRays = 490;  // rays per SM up to which a pipelined launch takes 168 registers, beyond them 128
+
+// Plasma warps of a pipelined block: one for one frequency; more frequencies make the plasma stage the longer one, so two
+// (up to 4) or four warps share them.
+template <int NF>
+constexpr int pipe_plasma_warps() {
+  return NF == 1 ? 1 : NF <= 4 ? 2 : 4;
+}
+
+template <Mode M, class PT, int NF, int kS, int kMinCtas>
+cudaError_t launch_pipe(const MarchArgs<typename Policy<M>::R, PT>& args, int sms, cudaStream_t stream,
+                        LaunchShape* shape) {
+  auto kern = k_march_pipe<M, PT, NF, kS, kMinCtas>;
+  constexpr int kBlock = 32 * (1 + kS);
+  cudaFuncAttributes fa;
+  cudaError_t e = cudaFuncGetAttributes(&fa, kern);
+  if (e != cudaSuccess) return e;
+  int bpsm = 0;
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bpsm, kern, kBlock, 0);
+  if (e != cudaSuccess) return e;
+  if (bpsm < 1) bpsm = 1;
+  const long long need = (args.njobs + 31) / 32;
+  long long grid = (long long)bpsm * sms;
+  if (grid > need) grid = need;
+  if (grid < 1) grid = 1;
+  shape->block = kBlock;
+  shape->grid = (int)grid;
+  shape->regs = fa.numRegs;
+  shape->local_bytes = (int)fa.localSizeBytes;
+  shape->blocks_per_sm = bpsm;
+  if (args.njobs <= 0) return cudaSuccess;
+  kern<<<(unsigned)grid, kBlock, 0, stream>>>(args);
+  return cudaGetLastError();
+}
+
 // Default variant per mode (measured on B200, 3 x 512^2 bench images): FP32 4 (128 registers, 16 warps); mixed with one
 // frequency slot 4 (128 registers, 140 bytes of spills: 474 ms vs 484 ms at 168 registers, 12 warps), mixed with more
 // slots 3 (4% faster than uncapped in 128-thread blocks); FP64 uncapped.
@@ -57,6 +110,17 @@ constexpr int default_blocks_per_sm() {
 template <Mode M, class PT, int NF>
 cudaError_t launch_nf(const MarchArgs<typename Policy<M>::R, PT>& args, int sms, int blocks_per_sm,
                       cudaStream_t stream, LaunchShape* shape) {
+  // a launch shape or refill policy named by the caller: always the plain kernel
+  if (blocks_per_sm <= 0 && args.default_schedule && args.njobs <= pipe_rays_per_sm<M, NF>() * sms) {
+    constexpr int kS = pipe_plasma_warps<NF>(), kThreads = 32 * (1 + kS);
+    if constexpr (M == Mode::kFP64) {
+      return launch_pipe<M, PT, NF, kS, 256 / kThreads>(args, sms, stream, shape);
+    } else {
+      return args.njobs <= (long long)kPipeWideRays * sms
+                 ? launch_pipe<M, PT, NF, kS, 384 / kThreads>(args, sms, stream, shape)
+                 : launch_pipe<M, PT, NF, kS, 512 / kThreads>(args, sms, stream, shape);
+    }
+  }
   if constexpr (M == Mode::kFP64) {
     (void)blocks_per_sm;
     return launch_mb<M, PT, NF, 128, 1>(args, sms, stream, shape);
