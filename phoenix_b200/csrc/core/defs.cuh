@@ -105,6 +105,15 @@ inline float fma_1(float a, float b, float c) { return a * b + c; }
 PHX_HD double mul_1(double a, double b) { return a * b; }
 PHX_HD double fma_1(double a, double b, double c) { return a * b + c; }
 
+// Whether the predicate holds in any of the lanes that are here (host: in the one ray).
+PHX_HD bool any_lane(bool p) {
+#if defined(__CUDA_ARCH__)
+  return __any_sync(__activemask(), p);
+#else
+  return p;
+#endif
+}
+
 template <class T>
 PHX_HD T sq(T x) {
   return x * x;

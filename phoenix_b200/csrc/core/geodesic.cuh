@@ -105,6 +105,23 @@ PHX_HD_OUTLINE StageDeriv<R> geodesic_accel_direct(StagePoint<R> p) {
   return o;
 }
 
+// What a step and a sample at its starting point share: the radius exp(x1) and, for the shifted stages, sin and cos of
+// x2 and of theta.  In FP64 an exp and two sincos cost about as much as a third of a stage; the mixed march took them again
+// for every sample.
+template <class R>
+struct StepTrig {
+  R e0, sx0, cx0, st0, ct0;
+
+  PHX_HD void at(R hs, R x2) {
+    sincos_t(x2, &sx0, &cx0);
+    // theta at the start, theta0 = x2 + (h/2) sin 2x2: each stage's theta follows from a small shift of it
+    sincos_t(x2 + R(0.5) * hs * (R(2) * sx0 * cx0), &st0, &ct0);
+  }
+  PHX_HD KerrPt<R> point(R a, R hs) const {
+    return kerr_point_theta<R, true>(a, hs, e0, R(2) * sx0 * cx0, (cx0 - sx0) * (cx0 + sx0), st0, ct0);
+  }
+};
+
 // One classical RK4 step of length dt.  Stage sums are kept as (d0 + d3) and (d1 + d2) so that the update
 // ((d0 + d3) + 2 (d1 + d2)) dt/6 needs two 12-vectors instead of four (kShift: one running sum).  The stage loop is deliberately not unrolled:
 // one copy of the stage body (metric, derivatives, both Christoffel contractions) keeps the march loop small enough
@@ -113,24 +130,18 @@ PHX_HD_OUTLINE StageDeriv<R> geodesic_accel_direct(StagePoint<R> p) {
 // step's starting point and short series of the stage offset (exp_small<7>, sincos_tiny: exact to rounding for
 // offsets up to kShiftMax), one exp and one sincos per step instead of four, and the geometry's reciprocals are the
 // Newton-refined FP64 ones (fastm::rcp_nr); a stage whose offset is larger evaluates the point directly.
-template <class R, bool kComp, int NS, bool kShift = false>
-PHX_HD void rk4_step(R a, R hs, GeoState<R, NS>& g, R dt) {
+template <class R, bool kComp, int NS, bool kShift = false, int kUnroll = 1>
+PHX_HD void rk4_step(R a, R hs, GeoState<R, NS>& g, R dt, const StepTrig<R>& tr) {
   constexpr bool kF = NS == 12;
   static_assert(!(kShift && kComp), "the shifted stages need an uncompensated state");
   const R pi_hi = R(kPi), pi_lo = R(kPi - (double)R(kPi));
   const bool south = kComp && g.hi[2] > R(kHalfPi);
-  R e0 = R(0), sx0 = R(0), cx0 = R(0), s2x0 = R(0), st0 = R(0), ct0 = R(0);
-  if constexpr (kShift) {
-    e0 = exp_t(g.hi[1]);
-    sincos_t(g.hi[2], &sx0, &cx0);
-    // theta at the start, theta0 = x2 + (h/2) sin 2x2: each stage's theta follows from a small shift of it
-    s2x0 = R(2) * sx0 * cx0;
-    sincos_t(g.hi[2] + R(0.5) * hs * s2x0, &st0, &ct0);
-  }
+  const R e0 = tr.e0, sx0 = tr.sx0, cx0 = tr.cx0, st0 = tr.st0, ct0 = tr.ct0;
+  const R s2x0 = R(2) * sx0 * cx0;
   R inc[NS], s03[NS], s12[NS];
 #pragma unroll
   for (int i = 0; i < NS; i++) inc[i] = R(0);
-#pragma unroll 1
+#pragma unroll kUnroll
   for (int q = 0; q < 4; q++) {
     R y[12];
 #pragma unroll
@@ -178,7 +189,8 @@ PHX_HD void rk4_step(R a, R hs, GeoState<R, NS>& g, R dt) {
         }
       }
     } else {
-      geodesic_accel<R, kF>(a, hs, y[1], y[2], y + 4, y + 8, d + 4, d + 8);
+      const R rs = q == 0 ? tr.e0 : exp_t(y[1]);
+      geodesic_accel_at<R, kF>(a, kerr_point_r(a, hs, rs, y[2]), y + 4, y + 8, d + 4, d + 8);
     }
     if (south) {
       d[2] = -d[2];
@@ -214,6 +226,15 @@ PHX_HD void rk4_step(R a, R hs, GeoState<R, NS>& g, R dt) {
       g.hi[i] += du;
     }
   }
+}
+
+// The step from its state alone.
+template <class R, bool kComp, int NS, bool kShift = false>
+PHX_HD void rk4_step(R a, R hs, GeoState<R, NS>& g, R dt) {
+  StepTrig<R> tr{};
+  tr.e0 = exp_t(geo_get<R, kComp>(g, 1));
+  if constexpr (kShift) tr.at(hs, g.hi[2]);
+  rk4_step<R, kComp, NS, kShift, 1>(a, hs, g, dt, tr);
 }
 
 // RAPTOR step size (negative: the ray runs backwards from the camera), capped by a quarter of the AMR cell.

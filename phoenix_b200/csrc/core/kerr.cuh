@@ -213,6 +213,26 @@ PHX_HD KerrPt<T> sample_point(T a, T hs, T r, T x2) {
   return p;
 }
 
+// The geometry at x2 + d for |d| <= kPointShift, from that at x2 (same radius): theta moves by theta' d + theta'' d^2 / 2,
+// and the terms of d^2 in sin and cos (5e-11) are below FP32's rounding.
+constexpr double kPointShift = 1e-5;
+
+template <class T>
+PHX_HD KerrPt<T> shifted_point(const KerrPt<T>& p, T a, T d) {
+  const T dth = d * (p.tp + T(0.5) * p.tpp * d);
+  KerrPt<T> o;
+  o.r = p.r;
+  o.s = p.s + p.c * dth;
+  o.c = p.c - p.s * dth;
+  o.s2 = o.s * o.s;
+  o.tp = p.tp + p.tpp * d;
+  o.tpp = p.tpp - T(4) * (p.tp - T(1)) * d;
+  o.sig = p.r * p.r + a * a * o.c * o.c;
+  o.isig = fastm::rcp(o.sig);
+  o.q = T(2) * p.r * o.isig;
+  return o;
+}
+
 // The metric of a plasma sample (cov_metric, contra_metric with the roundings spelled out; kGtt: g^tt with one rounding
 // instead of two).
 template <class T, bool kGtt>

@@ -193,20 +193,22 @@ PHX_HD int find_leaf(const SnapView<R, PT>& s, const R x[4], bool* scanned) {
 // Cell and trilinear weights of point x inside one leaf: weights measured from the block's lower corner and clamped at
 // the block faces (no ghost cells).  c: the lower corner cell (clamped into the block), del: weights of the upper
 // corners.
-template <class R, class PT, bool kFloorBy1000>
+template <class R, class PT, bool kFloorBy1000, bool kRcp = false>
 PHX_HD void cell_weights(const SnapView<R, PT>& s, int leaf, const R x[4], int c[3], R del[3]) {
 #pragma unroll
   for (int d = 0; d < 3; d++) {
     const R lb = ldg(s.lb + 3 * leaf + d), dx = ldg(s.dxc + 3 * leaf + d);
-    // FP32: one reciprocal per axis (rounding-level difference; the interpolant is continuous across cells)
-    const R idx = sizeof(R) == 4 ? fastm::rcp(dx) : R(0);
-    const R u = sizeof(R) == 4 ? mul_1(x[1 + d] - lb, idx) : (x[1 + d] - lb) / dx;
+    // FP32 and kRcp: one reciprocal per axis instead of two divisions (rounding-level difference; the interpolant is
+    // continuous across cells)
+    constexpr bool kByRcp = sizeof(R) == 4 || kRcp;
+    const R idx = kByRcp ? geo_rcp<R, kRcp>(dx) : R(0);
+    const R u = kByRcp ? mul_1(x[1 + d] - lb, idx) : (x[1 + d] - lb) / dx;
     c[d] = (int)u;
     if (c[d] >= s.nx[d]) c[d] = s.nx[d] - 1;
     if (c[d] < 0) c[d] = 0;  // unreachable for finite points of the leaf; keeps every gather inside the block
     const int ix = kFloorBy1000 ? (int)(u + R(1000)) - 1000 : (int)floor_t(u);
     const R off = x[1 + d] - fma_1(R(ix), dx, lb);
-    del[d] = (ix < 0) ? R(0) : (ix > s.nx[d] - 2) ? R(1) : (sizeof(R) == 4 ? mul_1(off, idx) : off / dx);
+    del[d] = (ix < 0) ? R(0) : (ix > s.nx[d] - 2) ? R(1) : (kByRcp ? mul_1(off, idx) : off / dx);
   }
 }
 
@@ -268,8 +270,9 @@ PHX_HD void interp_prims(const SnapView<R, PT>& s, int leaf, const R x[4], R q[k
 }
 
 // Fluid 4-velocity, magnetic 4-vector, |B| [G], n_e and Theta_e from the interpolated primitives; returns whether
-// the point emits (sampler.hpp:305-376).  g / u: metric at x.  kSpelled: B^2 with its roundings spelled out.
-template <class R, bool kSpelled>
+// the point emits (sampler.hpp:305-376).  g / u: metric at x.  kSig: which form of the roundings
+// (sample_point).
+template <class R, bool kSig>
 PHX_HD bool derive_fluid(const PlasmaView<R>& pv, R gam, R r, const Cov<R>& g, const Contra<R>& u, const R q[kNPrim],
                          Fluid<R>* fl) {
   const R smalll = R(1e-6);
@@ -300,18 +303,14 @@ PHX_HD bool derive_fluid(const PlasmaView<R>& pv, R gam, R r, const Cov<R>& g, c
   fl->B[1] = mul_1(fma_1(aB0, fl->U[1], Bp1), ilfac);
   fl->B[2] = mul_1(fma_1(aB0, fl->U[2], Bp2), ilfac);
   fl->B[3] = mul_1(fma_1(aB0, fl->U[3], Bp3), ilfac);
-  R bb2;
-  if constexpr (kSpelled) {
-    const R B0 = fl->B[0], B1 = fl->B[1], B2 = fl->B[2], B3 = fl->B[3];
-    bb2 = fma_1(mul_1(g.tt, B0), B0, mul_1(g.t1, R(2) * mul_1(B0, B1)));
-    bb2 = fma_1(g.t3, R(2) * mul_1(B0, B3), bb2);
-    bb2 = fma_1(mul_1(g.x11, B1), B1, bb2);
-    bb2 = fma_1(g.x13, R(2) * mul_1(B1, B3), bb2);
-    bb2 = fma_1(mul_1(g.x22, B2), B2, bb2);
-    bb2 = fma_1(mul_1(g.x33, B3), B3, bb2);
-  } else {
-    bb2 = dot(g, fl->B, fl->B);
-  }
+  const R B0 = fl->B[0], B1 = fl->B[1], B2 = fl->B[2], B3 = fl->B[3];
+  const R x22bb = mul_1(mul_1(g.x22, B2), B2);
+  R bb2 = fma_1(mul_1(g.tt, B0), B0, mul_1(g.t1, R(2) * mul_1(B0, B1)));
+  bb2 = fma_1(g.t3, R(2) * mul_1(B0, B3), bb2);
+  bb2 = fma_1(mul_1(g.x11, B1), B1, bb2);
+  bb2 = fma_1(g.x13, R(2) * mul_1(B1, B3), bb2);
+  bb2 = kSig ? fma_1(mul_1(g.x22, B2), B2, bb2) : bb2 + x22bb;
+  bb2 = fma_1(mul_1(g.x33, B3), B3, bb2);
   const R Bsq = fabs_t(bb2) + smalll;
   fl->Bmag = fastm::sqrt(Bsq) * pv.Bu;
   const R beta = fastm::div(uu * (gam - R(1)), R(0.5) * (Bsq + smalll));
@@ -327,6 +326,21 @@ PHX_HD bool derive_fluid(const PlasmaView<R>& pv, R gam, R r, const Cov<R>& g, c
     return false;
   }
   return true;
+}
+
+// B lowered, and its square: the plain contraction (kSig), or with the products that B^2 above shares with it rounded once.
+template <class R, bool kSig>
+PHX_HD R lower_field(const Cov<R>& g, const R B[4], R Bd[4]) {
+  if constexpr (kSig) {
+    symv(g, B, Bd);
+    return dot4(Bd, B);
+  } else {
+    Bd[0] = fma_1(g.t3, B[3], fma_1(g.t1, B[1], mul_1(g.tt, B[0])));
+    Bd[1] = fma_1(g.x13, B[3], fma_1(g.t1, B[0], mul_1(g.x11, B[1])));
+    Bd[2] = mul_1(g.x22, B[2]);
+    Bd[3] = fma_1(g.t3, B[0], mul_1(g.x13, B[1])) + mul_1(g.x33, B[3]);
+    return fma_1(Bd[3], B[3], fma_1(Bd[0], B[0], mul_1(Bd[1], B[1])) + mul_1(Bd[2], B[2]));
+  }
 }
 
 }  // namespace phx

@@ -33,8 +33,10 @@ PHX_HD void build_K(const Coeffs<R>& c, R c2, R s2, R K[4][4], R j[4]) {
   j[3] = c.jV;
 }
 
-// E = -h P^-1 K and S = h P^-1 j by Gauss-Jordan elimination with partial pivoting on [P | K | j].
-template <class R>
+// E = -h P^-1 K and S = h P^-1 j by Gauss-Jordan elimination on [P | K | j], with partial pivoting (kPivot) or without:
+// while the off-diagonal entries of each column of P sum to less than its diagonal entry, pivoting exchanges nothing and
+// the two give the same bits.
+template <class R, bool kPivot = true>
 PHX_HD void segment_operator(const R K[4][4], const R j[4], R h, R E[4][4], R S[4]) {
   R M[4][9];
   const R hh = R(0.5) * h;
@@ -50,7 +52,7 @@ PHX_HD void segment_operator(const R K[4][4], const R j[4], R h, R E[4][4], R S[
 #pragma unroll
   for (int c = 0; c < 4; c++) {
 #pragma unroll
-    for (int r = c + 1; r < 4; r++) {
+    for (int r = c + 1; kPivot && r < 4; r++) {
       const bool sw = fabs_t(M[r][c]) > fabs_t(M[c][c]);
 #pragma unroll
       for (int q = c; q < 9; q++) {

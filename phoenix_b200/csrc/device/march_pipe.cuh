@@ -73,7 +73,8 @@ __global__ void __launch_bounds__(32 * (1 + kS), kMinCtas)
         for (int c = 0; c < kPasses; c++) {
           bool sampled = false;
           if (live) {
-            live = ray.march(sg, A.rc, ctr, [&](const G* x, const G* k, const G* F, G r, G hl, int right) {
+            live = ray.template march<1>(sg, A.rc, ctr, [&](const G* x, const G* k, const G* F, G r, G hl, int right,
+                                                            const StepTrig<G>&) {
 #pragma unroll
               for (int i = 0; i < 3; i++) word[b][c][i][lane] = x[1 + i];
 #pragma unroll
@@ -137,7 +138,7 @@ __global__ void __launch_bounds__(32 * (1 + kS), kMinCtas)
 #pragma unroll
           for (int i = 0; i < 4; i++) F[i] = Geo::kWP ? G(0) : word[b][c][(Geo::kWP ? 0 : 9) + i][lane];
           ray.process_sample(A.snap, sg, A.rc, x, k, F, word[b][c][7][lane], word[b][c][8][lane],
-                             seed_leaf[b][c][lane], ctr, first);
+                             seed_leaf[b][c][lane], ctr, nullptr, first);
         }
         __syncwarp();
         if (!more[b]) break;
