@@ -4,14 +4,24 @@
 //   I, Q, U, V  summed over the pixels whose I+Q+U+V is finite, times the pixel solid angle and 1e23 (Jy);
 //   tau, tauF   means over the pixels whose six values sum to a finite number (0 when there are none).
 //
-// One thread-block cluster of kSpecCluster CTAs per frequency: each CTA sums a strided share of the pixels into
-// FP64 partials (warp shuffles, then its warps in a fixed order); CTA 0 of the cluster then reads the other CTAs'
-// partials through distributed shared memory, in rank order, and writes the record.  The result is deterministic
-// (no atomics) and nothing beyond the image and the output records is touched.
+// One thread-block cluster per frequency: each CTA sums a strided share of the pixels into FP64 partials (warp shuffles,
+// then its warps in a fixed order); CTA 0 of the cluster then reads the other CTAs' partials through distributed shared
+// memory, in rank order, and writes the record.  The result is deterministic (no atomics) and nothing beyond the image
+// and the output records is touched.
+//
+// The kernel is bound by what its SMs can read, so the cluster is the largest set of SMs that can add up partials without
+// scratch memory, 16 CTAs (8, the portable size, where the device cannot place 16), and a thread loads kSpecUnroll records
+// before it adds the first.  Measured (records of three images in turn): 1024^2 pixels, 4 frequencies 178 -> 94 us, 1
+// frequency 132 -> 35 us; 512^2, 3 frequencies 42 -> 25 us; 1400 x 1300, 6 frequencies 281 -> 131 us; images up to 300^2
+// stay at the launch's 13 to 17 us.  With several frequencies every lane's record is a cache line of its own and the L1's
+// tag lookups hold an SM at 33 GB/s; three lanes to a record (shuffled verdicts: 105 us for the first of these; staged
+// through shared memory: 86, but 55 and 31 us for the next two) did not pay.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <cmath>
+#include <map>
+#include <mutex>
 #include <stdexcept>
 
 #include "../host/render_setup.hpp"
@@ -22,7 +32,8 @@ using namespace phx_capi;
 
 namespace {
 
-constexpr int kSpecCluster = 8;
+constexpr int kSpecCluster = 16, kSpecClusterPortable = 8;
+constexpr int kSpecUnroll = 6;  // records a thread has in flight
 constexpr int kSpecThreads = 512;
 constexpr int kSpecWarps = kSpecThreads / 32;
 
@@ -43,32 +54,45 @@ __device__ __forceinline__ unsigned long long warp_sum(unsigned long long v) {
   return v;
 }
 
-__global__ void __cluster_dims__(kSpecCluster, 1, 1) __launch_bounds__(kSpecThreads)
+__global__ void __launch_bounds__(kSpecThreads)
     k_spectrum(const double2* __restrict__ res, long long npix, int nfreqs, double jy_per_unit,
                PhxSpectrum* __restrict__ out) {
   __shared__ SpecPart warp_part[kSpecWarps];
   __shared__ SpecPart cta_part;
   cg::cluster_group cluster = cg::this_cluster();
-  const unsigned rank = cluster.block_rank();
+  const unsigned rank = cluster.block_rank(), ncta = cluster.num_blocks();
   const int f = blockIdx.y;
   double s[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
   unsigned long long nflux = 0, ntau = 0;
-  const long long stride = (long long)kSpecCluster * kSpecThreads;
-  for (long long p = (long long)rank * kSpecThreads + threadIdx.x; p < npix; p += stride) {
-    const double2* r = res + ((size_t)p * nfreqs + f) * 3;  // one 48-byte record: three 16-byte loads
-    const double2 iq = __ldg(r), uv = __ldg(r + 1), tt = __ldg(r + 2);
-    const double stokes = iq.x + iq.y + uv.x + uv.y;
-    if (isfinite(stokes)) {
-      s[0] += iq.x;
-      s[1] += iq.y;
-      s[2] += uv.x;
-      s[3] += uv.y;
-      nflux++;
+  const long long stride = (long long)ncta * kSpecThreads;
+  for (long long p0 = (long long)rank * kSpecThreads + threadIdx.x; p0 < npix; p0 += kSpecUnroll * stride) {
+    double2 v[kSpecUnroll][3];
+#pragma unroll
+    for (int u = 0; u < kSpecUnroll; u++) {
+      const long long p = p0 + u * stride;
+      if (p < npix) {
+        const double2* r = res + ((size_t)p * nfreqs + f) * 3;  // one 48-byte record: three 16-byte loads
+#pragma unroll
+        for (int w = 0; w < 3; w++) v[u][w] = __ldg(r + w);
+      }
     }
-    if (isfinite(stokes + tt.x + tt.y)) {
-      s[4] += tt.x;
-      s[5] += tt.y;
-      ntau++;
+#pragma unroll
+    for (int u = 0; u < kSpecUnroll; u++) {
+      if (p0 + u * stride >= npix) break;
+      const double2 iq = v[u][0], uv = v[u][1], tt = v[u][2];
+      const double stokes = iq.x + iq.y + uv.x + uv.y;
+      if (isfinite(stokes)) {
+        s[0] += iq.x;
+        s[1] += iq.y;
+        s[2] += uv.x;
+        s[3] += uv.y;
+        nflux++;
+      }
+      if (isfinite(stokes + tt.x + tt.y)) {
+        s[4] += tt.x;
+        s[5] += tt.y;
+        ntau++;
+      }
     }
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -95,7 +119,7 @@ __global__ void __cluster_dims__(kSpecCluster, 1, 1) __launch_bounds__(kSpecThre
   cluster.sync();  // every CTA's partial is in its shared memory
   if (rank == 0 && threadIdx.x == 0) {
     SpecPart t = cta_part;
-    for (unsigned c = 1; c < kSpecCluster; c++) {
+    for (unsigned c = 1; c < ncta; c++) {
       const SpecPart* o = cluster.map_shared_rank(&cta_part, c);
       for (int q = 0; q < 6; q++) t.s[q] += o->s[q];
       t.n[0] += o->n[0];
@@ -112,6 +136,33 @@ __global__ void __cluster_dims__(kSpecCluster, 1, 1) __launch_bounds__(kSpecThre
   cluster.sync();  // CTA 0 has read the others' shared memory before they exit
 }
 
+// Whether the current device can place a cluster of kSpecCluster CTAs of k_spectrum (16 is beyond the portable 8).
+bool wide_clusters() {
+  int dev = 0;
+  ck(cudaGetDevice(&dev), "cudaGetDevice");
+  static std::mutex mu;
+  static std::map<int, bool> known;  // a property of the device and the kernel
+  std::lock_guard<std::mutex> lock(mu);
+  const auto it = known.find(dev);
+  if (it != known.end()) return it->second;
+  bool ok = cudaFuncSetAttribute(k_spectrum, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+  if (ok) {
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim = {(unsigned)kSpecCluster, 1, 1};
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kSpecCluster);
+    cfg.blockDim = dim3(kSpecThreads);
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    ok = cudaOccupancyMaxActiveClusters(&n, k_spectrum, &cfg) == cudaSuccess && n >= 1;
+  }
+  if (!ok) cudaGetLastError();
+  known[dev] = ok;
+  return ok;
+}
+
 }  // namespace
 
 namespace phx_capi {
@@ -120,8 +171,17 @@ void launch_spectrum(const PhxRenderParams& p, const PhxFreqOut* d_res, PhxSpect
   if ((reinterpret_cast<uintptr_t>(d_res) & 15u) != 0) throw std::invalid_argument("d_res must be 16-byte aligned");
   const long long npix = (long long)p.img_width * p.img_height;
   const double jy = phx::pixel_solid_angle(p) * phx::cgs::jansky;
-  const dim3 grid(kSpecCluster, p.nfreqs), block(kSpecThreads);
-  k_spectrum<<<grid, block, 0, st>>>(reinterpret_cast<const double2*>(d_res), npix, p.nfreqs, jy, d_spec);
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim = {(unsigned)(wide_clusters() ? kSpecCluster : kSpecClusterPortable), 1, 1};
+  cudaLaunchConfig_t cfg = {};
+  cfg.blockDim = dim3(kSpecThreads);
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  cfg.gridDim = dim3(attr.val.clusterDim.x, p.nfreqs);
+  ck(cudaLaunchKernelEx(&cfg, k_spectrum, reinterpret_cast<const double2*>(d_res), npix, (int)p.nfreqs, jy, d_spec),
+     "spectrum launch");
   ck(cudaGetLastError(), "spectrum launch");
 }
 
