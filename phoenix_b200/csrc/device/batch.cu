@@ -24,6 +24,7 @@ using namespace phx_capi;
 
 struct PhxBatch {
   int device = 0, sms = 0;
+  std::string device_name;  // asked once: the property query takes milliseconds, at times hundreds
   int32_t precision = PHX_PREC_FP32;
   int nf_slots = 1;
   std::vector<PhxRenderParams> params;
@@ -282,6 +283,7 @@ PhxBatch* create_batch(const PhxBatchItem* items, int32_t nitems, const PhxBatch
     maxf = std::max(maxf, (int)it.params.nfreqs);
     f64prims = f64prims && it.snapshot->prim_d;
     b->sms = it.snapshot->sms;
+    b->device_name = it.snapshot->device_name;
   }
   b->nf_slots = maxf <= 1 ? 1 : maxf <= 4 ? 4 : phx::kMaxFreqs;
   if (b->nf_slots > 4 && b->precision != PHX_PREC_FP32)
@@ -450,9 +452,7 @@ int phx_batch_result(PhxBatch* b, int32_t item, PhxFreqOut* res, PhxRenderInfo* 
       ck(cudaMemcpy(c, b->item_ctr + (size_t)phx::kItemCounters * item, sizeof c, cudaMemcpyDeviceToHost),
          "D2H counters");
       std::memset(info, 0, sizeof *info);
-      cudaDeviceProp prop;
-      ck(cudaGetDeviceProperties(&prop, b->device), "cudaGetDeviceProperties");
-      std::snprintf(info->device, sizeof info->device, "%.200s (sm_%d%d)", prop.name, prop.major, prop.minor);
+      std::snprintf(info->device, sizeof info->device, "%s", b->device_name.c_str());
       info->sms = b->sms;
       info->blocks = b->lshape.grid;
       info->block = b->lshape.block;

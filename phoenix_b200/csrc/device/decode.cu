@@ -49,11 +49,15 @@ __global__ void __launch_bounds__(128) k_decode(const __grid_constant__ DecodeAr
 
 namespace phx_capi {
 
+// Bytes of a pinned buffer.  Pinning costs more than reading: with two buffers of 64 MB a 122 MB dump loaded in 100 ms (at
+// times a second), with two of 8 MB in 30; a 1.37 GB dump in 300 and 180.
+constexpr size_t kDecodeChunkBytes = 8u << 20;
+
 // Decodes the dump's cells into s's device primitive pool (allocated, not yet filled); returns the seconds spent.
 double gpu_decode(PhxSnapshot* s, const std::string& dump, const phx::HostSnapshot& meta, int bpol) {
   const auto t0 = std::chrono::steady_clock::now();
   const size_t leaf_doubles = (size_t)meta.nwini * meta.cells;
-  const int chunk = (int)std::max<size_t>(1, std::min<size_t>(meta.nleafs, (64u << 20) / (leaf_doubles * 8)));
+  const int chunk = (int)std::max<size_t>(1, std::min<size_t>(meta.nleafs, kDecodeChunkBytes / (leaf_doubles * 8)));
   double* host[2] = {nullptr, nullptr};
   double* dev[2] = {nullptr, nullptr};
   cudaStream_t st[2] = {nullptr, nullptr};
