@@ -123,9 +123,10 @@ struct StepTrig {
 };
 
 // One classical RK4 step of length dt.  Stage sums are kept as (d0 + d3) and (d1 + d2) so that the update
-// ((d0 + d3) + 2 (d1 + d2)) dt/6 needs two 12-vectors instead of four (kShift: one running sum).  The stage loop is deliberately not unrolled:
-// one copy of the stage body (metric, derivatives, both Christoffel contractions) keeps the march loop small enough
-// for the instruction cache, which four unrolled copies overflow.
+// ((d0 + d3) + 2 (d1 + d2)) dt/6 needs two 12-vectors instead of four (kShift: one running sum).
+// kUnroll: copies of the stage body in the loop.  More copies know which sums a stage adds to, and fetch more code: FP32
+// gains with four (GeoRay::march's callers), the FP64 stages and the pipelined geodesic warps with one.  The stage
+// increments are rounded before they are added (mul_1), so that every count gives the same bits.
 // kShift (uncompensated state only; the mixed mode's FP64 geodesic): each stage's exp(x1) and sincos(x2) come from the
 // step's starting point and short series of the stage offset (exp_small<7>, sincos_tiny: exact to rounding for
 // offsets up to kShiftMax), one exp and one sincos per step instead of four, and the geometry's reciprocals are the
@@ -213,7 +214,7 @@ PHX_HD void rk4_step(R a, R hs, GeoState<R, NS>& g, R dt, const StepTrig<R>& tr)
     if (q < 3) {
       const R wdt = (q == 2 ? R(1) : R(0.5)) * dt;
 #pragma unroll
-      for (int i = 0; i < NS; i++) inc[i] = wdt * d[i];
+      for (int i = 0; i < NS; i++) inc[i] = mul_1(wdt, d[i]);
     }
   }
   const R dt6 = dt / R(6);

@@ -525,11 +525,14 @@ struct Ray : GeoRay<M, PT>, PlasmaRay<M, PT, NF, typename RayStore<M, PT, NF>::A
     Plasma::start(st.kappa);
   }
 
+  // kUnroll: copies of the FP32 RK4 stage.  Four: a 512^2 image 74.2 -> 70.0 ms (two: 71.1), 1024^2 with 3 frequencies 382
+  // -> 376; the queue kernel, whose lanes read their image's constants from memory, takes two (8 served requests 86.5 ms,
+  // with four 89.1).  Mixed: two are 3% slower than one.
+  template <int kUnroll = 4>
   PHX_HD bool advance(const SnapView<R, PT>& s, const SnapView<double, PT>& sd, const RenderConsts<R>& rc,
                       RayCounters& ctr) {
     const SnapView<G, PT>& sg = Geo::geo_view(s, sd);
-    // FP32: two stages per round of the RK4 loop are 1.4% faster on a 512^2 image (mixed 3% slower)
-    return Geo::template march<M == Mode::kFP32 ? 2 : 1>(
+    return Geo::template march<M == Mode::kFP32 ? kUnroll : 1>(
         sg, rc, ctr, [&](const G* x, const G* k, const G* F, G r, G hl, int right, const StepTrig<G>& tr) {
           if constexpr (Geo::kShift) {  // the step's own sines and cosines
             const KerrPt<G> own = tr.point(sg.a, sg.hs);

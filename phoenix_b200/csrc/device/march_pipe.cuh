@@ -8,7 +8,8 @@
 // The arithmetic of a ray is the plain kernel's (march.cuh), so are its results.
 //
 // Chunks are double-buffered; one barrier of the block per chunk hands a filled buffer over and gets the other one back
-// (4 passes of FP32 points, 2 of FP64 ones: 10 to 14 KB of shared memory a block).
+// (8 passes of FP32 points, 2 of FP64 ones: 10 to 21 KB of shared memory a block; FP32 with 4: 1 to 2% slower, FP64 with 4:
+// the same).
 //
 // A 64^2 FP32 image takes 10.4 ms against the plain kernel's 15.9 (about 2,040 cycles a pass against 3,215; a march
 // without any samples 8.6 ms).  Unrolling the RK4 stages for more parallelism inside the geodesic warp was slower at
@@ -26,7 +27,7 @@ __global__ void __launch_bounds__(32 * (1 + kS), kMinCtas)
   using R = typename Policy<M>::R;
   using G = typename Policy<M>::G;
   constexpr unsigned kFull = 0xffffffffu;
-  constexpr int kPasses = sizeof(G) == 4 ? 4 : 2;  // passes of a chunk
+  constexpr int kPasses = sizeof(G) == 4 ? 8 : 2;  // passes of a chunk
   constexpr int kWords = Geo::kWP ? 9 : 13;        // x1..x3, k, r, step length (FP64: and F)
   __shared__ G word[2][kPasses][kWords][32];
   __shared__ int32_t seed_leaf[2][kPasses][32];

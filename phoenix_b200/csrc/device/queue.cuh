@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks)
     idle = 0;
     for (int it = 0; it < A.period; it++) {
       if (live) {
-        live = ray.advance(d->snap, d->snap_d, d->rc, ctr);
+        live = ray.template advance<2>(d->snap, d->snap_d, d->rc, ctr);
         if (!live) {
           ray.write(d->out, d->rc.nfreqs);
           if (d->pixstats) {
