@@ -288,15 +288,18 @@ struct GeoRay : RayTypes<M, PT> {
 
 // The plasma stage of a ray: its Walker-Penrose constant and its transfer records (AccStore).  It takes every kStride-th
 // frequency from `first` on (all of them: 1, 0), and keeps a record for each of those it takes.
-template <Mode M, class PT, int NF, class AccStore, int kStride = 1>
+template <Mode M, class PT, int NF, class AccStore, int kStride = 1, bool kQueue = false>
 struct PlasmaRay : RayTypes<M, PT> {
   using T = RayTypes<M, PT>;
   using R = typename T::R;
   using G = typename T::G;
   using T::kComp, T::kMixed, T::kWP;
-  // the one-slot mixed kernels round the sample's Sigma and B^2 the other way than the rest (sample_point, derive_fluid),
-  // as they always have: a sample on an emission cut or next to a field line turns on the last bit
-  static constexpr bool kSig = !(kMixed && NF == 1);
+  // Which way the sample's Sigma and B^2 (kSig: sample_point, derive_fluid) and g^tt (kGtt: sample_metric) are rounded: the
+  // mixed kernels of one slot (not the queue's) have always had another form of the first two than the rest, those of up to
+  // 4 slots (the queue's: of one) of the last, and a sample on an emission cut or next to a field line turns on the last
+  // bit.
+  static constexpr bool kSig = !(kMixed && NF == 1 && !kQueue);
+  static constexpr bool kGtt = !(kMixed && NF <= (kQueue ? 1 : 4));
 
   R kappa[2];  // Walker-Penrose constant of (k, F1) (kWP)
   int nplasma, bad;
@@ -346,7 +349,7 @@ struct PlasmaRay : RayTypes<M, PT> {
     const KerrPt<R> p = sample_point<R, kSig>(s.a, s.hs, rx, x2w);
     Cov<R> g;
     Contra<R> u;
-    sample_metric<R, !kMixed || (NF > 4)>(p, s.a, &g, &u);
+    sample_metric<R, kGtt>(p, s.a, &g, &u);
     Fluid<R> fl;
     if (!derive_fluid<R, kSig>(rc.pv, s.gam, rx, g, u, q, &fl)) return;
     if (!(r < rc.template steps_in<G>().rt_outer)) return;
@@ -503,11 +506,11 @@ struct RayStore {
   using AccStore = std::conditional_t<kAccShared, AccShared<R, T::kMixed, NF>, AccRegs<R, T::kMixed, NF>>;
 };
 
-// One ray, marched and sampled by one lane.
-template <Mode M, class PT, int NF>
-struct Ray : GeoRay<M, PT>, PlasmaRay<M, PT, NF, typename RayStore<M, PT, NF>::AccStore> {
+// One ray, marched and sampled by one lane (kQueue: of the queue kernel).
+template <Mode M, class PT, int NF, bool kQueue = false>
+struct Ray : GeoRay<M, PT>, PlasmaRay<M, PT, NF, typename RayStore<M, PT, NF>::AccStore, 1, kQueue> {
   using Geo = GeoRay<M, PT>;
-  using Plasma = PlasmaRay<M, PT, NF, typename RayStore<M, PT, NF>::AccStore>;
+  using Plasma = PlasmaRay<M, PT, NF, typename RayStore<M, PT, NF>::AccStore, 1, kQueue>;
   using R = typename Geo::R;
   using G = typename Geo::G;
   static constexpr size_t kSmemPerThread = RayStore<M, PT, NF>::AccStore::kSmemPerThread;

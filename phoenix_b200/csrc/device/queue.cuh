@@ -90,7 +90,7 @@ template <Mode M, class PT, int NF, int kBlock, int kMinBlocks>
 __global__ void __launch_bounds__(kBlock, kMinBlocks)
     k_queue(const __grid_constant__ QueueArgs<typename Policy<M>::R, PT> A) {
   using R = typename Policy<M>::R;
-  using RayT = Ray<M, PT, NF>;
+  using RayT = Ray<M, PT, NF, true>;
   using Item = ItemDesc<R, PT>;
   constexpr unsigned kFull = 0xffffffffu;
   const unsigned lane = threadIdx.x & 31u;
