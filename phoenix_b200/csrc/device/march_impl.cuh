@@ -46,20 +46,21 @@ cudaError_t launch_mb(const MarchArgs<typename Policy<M>::R, PT>& args, int sms,
 
 // The pipelined kernel (march_pipe.cuh) takes the launches of few rays per SM.  Its blocks hold one ray per lane of their
 // geodesic warp only, so 168 registers leave room for 192 rays an SM (128: 256) against the plain kernel's 512: it wins
-// while a launch is as long as its longest rays, and loses once the rays fill the chip several times over.  ms of one
-// image at 20 / 75 deg, pipelined against plain (96^3-base snapshot; the same bits for FP64):
-//   FP32, 1 frequency:   64^2 10.5 / 10.1 against 16.2 / 16.0;  128^2 15.1 / 11.7 : 21.5 / 16.3;  200^2 17.8 / 14.2 : 23.9 / 20.6;
-//     256^2 (443 rays an SM) 20.3 / 20.8 : 26.8 / 30.3;  320^2 (692) 29.5 / 25.6, 128 registers 27.4 / 24.2 : 29.2 / 27.0;
-//     400^2 (1081) 128 registers 41.1 / 35.9 : 42.8 / 32.8;  512^2 65.6 / 56.4 : 48.4 / 42.3
-//   FP32, 3 frequencies: 128^2 18.4 / 17.5 : 22.4 / 20.0;  256^2 35.6 / 33.2, 128 registers 33.9 / 31.7 : 31.6 / 37.6;
-//     400^2 79.0 / 72.8 : 51.6 / 40.7
-//   FP32, 8 frequencies: 64^2 13.2 / 12.3 : 29.1 / 24.7;  128^2 18.2 / 16.4 : 27.1 / 27.8;  200^2 (270) 34.7 / 32.0 : 39.7 / 35.2
-//   mixed, 1 frequency:  64^2 14.8 / 15.5 : 24.9 / 25.2;  256^2 30.9 / 32.5 : 41.3 / 47.7;  320^2 128 registers 40.7 / 34.5 :
-//     45.7 / 42.4;  400^2 61.4 / 52.4 : 66.8 / 48.8;  3 frequencies, 333 x 217 (488) 54.7 / 49.1 : 60.5 / 62.7
-//   FP64, 1 frequency:   64^2 30.2 / 30.8 : 45.9 / 45.9;  200^2 (270) 69.0 / 55.7 : 79.8 / 68.2;  256^2 95.9 / 81.7 : 82.6 / 93.5
+// while a launch is as long as its longest rays, and loses once the rays fill the chip several times over, the sooner the
+// longer the plasma stage is.  Plain kernel's time over the pipelined one's at 20 / 75 deg (96 x 48 x 48-base snapshot), by
+// rays per SM:
+//   FP32, 1 frequency: 28 1.6 / 1.6, 442 1.22 / 1.34, 529 1.10 / 1.17, 691 0.97 / 1.00;  2: 442 1.07 / 1.24;  3: 270 1.22 / 1.16,
+//     389 1.12 / 1.18, 492 0.91 / 0.95;  4: 492 1.09 / 1.15;  5: 389 0.94 / 0.94;  8: 172 1.58 / 1.60, 270 1.40 / 1.32;  32: 27 3.1 / 3.3, 270 2.0 / 1.8
+//   mixed, 1: 28 1.7 / 1.7, 442 1.33 / 1.52, 691 1.11 / 1.19;  2: 442 1.08 / 1.48;  3: 270 1.30 / 1.30, 492 0.90 / 0.97;  8: 67
+//     1.72 / 1.90, 270 1.16 / 1.12
+//   FP64, 1: 110 1.28 / 1.19, 297 1.21 / 1.36;  3: 67 1.26 / 1.23, 110 1.09 / 1.08, 172 0.96 / 0.98, 270 0.72 / 0.70;  8: 110 1.38 /
+//     1.53, 270 0.92 / 0.82
+// Odd widths put a column of rays over the poles that all take the most steps there are, and gain more: FP32, 351 x 333 (789)
+// 1.13 / 1.14, 3 frequencies 271 x 269 (492) 1.11 / 1.23; mixed 1.26 / 1.32 and 1.12 / 1.13.  The limits lie between the two.
 template <Mode M, int NF>
 constexpr long long pipe_rays_per_sm() {
-  return M == Mode::kFP64 || NF > 4 ? 300 : NF > 1 ? 500 : 700;
+  return M == Mode::kFP64 ? (NF == 1 ? 300 : NF <= 4 ? 140 : 180)
+                          : NF == 1 ? (M == Mode::kFP32 ? 700 : 850) : NF <= 4 ? 500 : (M == Mode::kFP32 ? 320 : 300);
 }
 constexpr int kPipeWideRays = 490;  // rays per SM up to which a pipelined launch takes 168 registers, beyond them 128
 
