@@ -104,7 +104,7 @@ typedef struct {
   int32_t blocks_per_sm; /* register-cap variant, as resident warps per SM / 4 (1: up to 255 registers in 128-thread
                             blocks; 3: 168 registers, 4: 128, as one 384 / 512-thread block per SM when the job list
                             fills every SM, else as 128-thread blocks); 0 = default (FP32 4; mixed 4 with one frequency, else 3;
-                            FP64 1) */
+                            FP64 1; with the default period and refill, a small launch runs as a pipeline of warps) */
   int32_t refill_lanes; /* a warp takes new jobs early, before the period ends, once this many of its 32 lanes have
                            finished (checked every 64 passes); 1..32, 0 = default (32: when the warp is empty) */
 } PhxRenderParams;

@@ -364,7 +364,7 @@ PhxBatch* create_batch(const PhxBatchItem* items, int32_t nitems, const PhxBatch
     nrec += (size_t)npix * p.nfreqs;
   }
   b->nrecords = nrec;
-  // tiles: the largest images first unless the caller keeps its order
+  // tiles, the largest images first unless the caller keeps its order; place_tiles then orders them by band
   std::vector<int32_t> order(nitems);
   std::iota(order.begin(), order.end(), 0);
   if (!o.keep_order)
