@@ -11,7 +11,7 @@
 //
 // The kernel is bound by what its SMs can read, so the cluster is the largest set of SMs that can add up partials without
 // scratch memory, 16 CTAs (8, the portable size, where the device cannot place 16), and a thread loads kSpecUnroll records
-// before it adds the first.  Measured (records of three images in turn): 1024^2 pixels, 4 frequencies 178 -> 94 us, 1
+// before it adds the first.  Measured (records of three images in turn): 1024^2 pixels, 4 frequencies 178 -> 96 us, 1
 // frequency 132 -> 35 us; 512^2, 3 frequencies 42 -> 25 us; 1400 x 1300, 6 frequencies 281 -> 131 us; images up to 300^2
 // stay at the launch's 13 to 17 us.  With several frequencies every lane's record is a cache line of its own and the L1's
 // tag lookups hold an SM at 33 GB/s; three lanes to a record (shuffled verdicts: 105 us for the first of these; staged
@@ -37,10 +37,30 @@ constexpr int kSpecUnroll = 6;  // records a thread has in flight
 constexpr int kSpecThreads = 512;
 constexpr int kSpecWarps = kSpecThreads / 32;
 
+// Sums of a warp, a CTA or the cluster.  From the warps up they are compensated: s + e is the sum, e what the additions
+// to s rounded off.  Every addition there rounds at the size of the total, and the 15 CTAs after the first alone put
+// 1e-16 on it; the threads' and the shuffles' roundings are of parts and average out.  Mean error of 24 images' totals against
+// an exact sum 9e-18 (8 CTAs without it: 6.7e-17); 2 us of 96.
 struct SpecPart {
-  double s[6];              // I, Q, U, V, tau, tauF
+  double s[6], e[6];        // I, Q, U, V, tau, tauF
   unsigned long long n[2];  // pixels in the flux sum, in the optical-depth means
 };
+
+// a += b (Knuth's two-sum; an infinite sum leaves a NaN in e, which total() drops).
+__device__ __forceinline__ void add_part(SpecPart& a, const SpecPart& b) {
+#pragma unroll
+  for (int q = 0; q < 6; q++) {
+    const double x = a.s[q], y = b.s[q], t = x + y, z = t - x;
+    a.s[q] = t;
+    a.e[q] += b.e[q] + ((x - (t - z)) + (y - z));
+  }
+  a.n[0] += b.n[0];
+  a.n[1] += b.n[1];
+}
+__device__ __forceinline__ double total(const SpecPart& a, int q) {
+  const double t = a.s[q] + a.e[q];
+  return isfinite(t) ? t : a.s[q];
+}
 
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
@@ -102,33 +122,27 @@ __global__ void __launch_bounds__(kSpecThreads)
   ntau = warp_sum(ntau);
   if (lane == 0) {
 #pragma unroll
-    for (int q = 0; q < 6; q++) warp_part[warp].s[q] = s[q];
+    for (int q = 0; q < 6; q++) {
+      warp_part[warp].s[q] = s[q];
+      warp_part[warp].e[q] = 0.0;
+    }
     warp_part[warp].n[0] = nflux;
     warp_part[warp].n[1] = ntau;
   }
   __syncthreads();
   if (threadIdx.x == 0) {
     SpecPart t = warp_part[0];
-    for (int w = 1; w < kSpecWarps; w++) {
-      for (int q = 0; q < 6; q++) t.s[q] += warp_part[w].s[q];
-      t.n[0] += warp_part[w].n[0];
-      t.n[1] += warp_part[w].n[1];
-    }
+    for (int w = 1; w < kSpecWarps; w++) add_part(t, warp_part[w]);
     cta_part = t;
   }
   cluster.sync();  // every CTA's partial is in its shared memory
   if (rank == 0 && threadIdx.x == 0) {
     SpecPart t = cta_part;
-    for (unsigned c = 1; c < ncta; c++) {
-      const SpecPart* o = cluster.map_shared_rank(&cta_part, c);
-      for (int q = 0; q < 6; q++) t.s[q] += o->s[q];
-      t.n[0] += o->n[0];
-      t.n[1] += o->n[1];
-    }
+    for (unsigned c = 1; c < ncta; c++) add_part(t, *cluster.map_shared_rank(&cta_part, c));
     PhxSpectrum rec;
-    for (int q = 0; q < 4; q++) rec.IQUV[q] = t.s[q] * jy_per_unit;
-    rec.tau_mean = t.n[1] ? t.s[4] / (double)t.n[1] : 0.0;
-    rec.tauF_mean = t.n[1] ? t.s[5] / (double)t.n[1] : 0.0;
+    for (int q = 0; q < 4; q++) rec.IQUV[q] = total(t, q) * jy_per_unit;
+    rec.tau_mean = t.n[1] ? total(t, 4) / (double)t.n[1] : 0.0;
+    rec.tauF_mean = t.n[1] ? total(t, 5) / (double)t.n[1] : 0.0;
     rec.n_flux = (int64_t)t.n[0];
     rec.n_tau = (int64_t)t.n[1];
     out[f] = rec;
