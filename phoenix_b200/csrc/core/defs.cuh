@@ -105,6 +105,24 @@ inline float fma_1(float a, float b, float c) { return a * b + c; }
 PHX_HD double mul_1(double a, double b) { return a * b; }
 PHX_HD double fma_1(double a, double b, double c) { return a * b + c; }
 
+// FP64 operations with the rounding spelled out, on the device as on the host: a product and a sum that are never
+// contracted, and a fused one.  The mixed geodesic is written in them (geodesic_accel_1 says why).
+PHX_HD double dmul_1(double a, double b) {
+#if defined(__CUDA_ARCH__)
+  return __dmul_rn(a, b);
+#else
+  return a * b;
+#endif
+}
+PHX_HD double dadd_1(double a, double b) {
+#if defined(__CUDA_ARCH__)
+  return __dadd_rn(a, b);
+#else
+  return a + b;
+#endif
+}
+PHX_HD double dfma_1(double a, double b, double c) { return fma(a, b, c); }
+
 // Whether the predicate holds in any of the lanes that are here (host: in the one ray).
 PHX_HD bool any_lane(bool p) {
 #if defined(__CUDA_ARCH__)

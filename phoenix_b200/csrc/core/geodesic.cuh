@@ -65,10 +65,10 @@ template <class T, int N = 11>
 PHX_HD T exp_small(T d) {
   if constexpr (N == 7) {
     // Estrin's form: three levels of independent products instead of a seven-deep Horner chain
-    const T d2 = d * d, d4 = d2 * d2;
-    const T q0 = (T(1) + d) + d2 * (T(1.0 / 2.0) + d * T(1.0 / 6.0));
-    const T q1 = (T(1.0 / 24.0) + d * T(1.0 / 120.0)) + d2 * (T(1.0 / 720.0) + d * T(1.0 / 5040.0));
-    return q0 + d4 * q1;
+    const T d2 = dmul_1(d, d), d4 = dmul_1(d2, d2);
+    const T q0 = dfma_1(d2, dfma_1(d, 1.0 / 6.0, 1.0 / 2.0), dadd_1(1.0, d));
+    const T q1 = dfma_1(d2, dfma_1(d, 1.0 / 5040.0, 1.0 / 720.0), dfma_1(d, 1.0 / 120.0, 1.0 / 24.0));
+    return dfma_1(d4, q1, q0);
   } else {
     T e = T(1);
 #pragma unroll
@@ -106,8 +106,8 @@ PHX_HD_OUTLINE StageDeriv<R> geodesic_accel_direct(StagePoint<R> p) {
 }
 
 // What a step and a sample at its starting point share: the radius exp(x1) and, for the shifted stages, sin and cos of
-// x2 and of theta.  In FP64 an exp and two sincos cost about as much as a third of a stage; the mixed march took them again
-// for every sample.
+// x2 and of theta.  In FP64 an exp and two sincos cost about as much as a third of a stage; the mixed march took exp and
+// sincos(x2) again for every sample.
 template <class R>
 struct StepTrig {
   R e0, sx0, cx0, st0, ct0;
@@ -115,11 +115,12 @@ struct StepTrig {
   PHX_HD void at(R hs, R x2) {
     sincos_t(x2, &sx0, &cx0);
     // theta at the start, theta0 = x2 + (h/2) sin 2x2: each stage's theta follows from a small shift of it
-    sincos_t(x2 + R(0.5) * hs * (R(2) * sx0 * cx0), &st0, &ct0);
+    sincos_t(dfma_1(0.5 * hs, s2x0(), x2), &st0, &ct0);
   }
-  PHX_HD KerrPt<R> point(R a, R hs) const {
-    return kerr_point_theta<R, true>(a, hs, e0, R(2) * sx0 * cx0, (cx0 - sx0) * (cx0 + sx0), st0, ct0);
-  }
+  PHX_HD R s2x0() const { return dmul_1(2.0 * sx0, cx0); }
+  // The step's starting point for its sample.  sin theta by angle addition: next to the south pole, sincos(theta0) has only
+  // the digits that theta0 has.
+  PHX_HD KerrPt<R> point(R a, R hs, R x2) const { return kerr_point_rsc(a, hs, e0, x2, sx0, cx0); }
 };
 
 // One classical RK4 step of length dt.  Stage sums are kept as (d0 + d3) and (d1 + d2) so that the update
@@ -130,15 +131,14 @@ struct StepTrig {
 // kShift (uncompensated state only; the mixed mode's FP64 geodesic): each stage's exp(x1) and sincos(x2) come from the
 // step's starting point and short series of the stage offset (exp_small<7>, sincos_tiny: exact to rounding for
 // offsets up to kShiftMax), one exp and one sincos per step instead of four, and the geometry's reciprocals are the
-// Newton-refined FP64 ones (fastm::rcp_nr); a stage whose offset is larger evaluates the point directly.
+// Newton-refined FP64 ones (fastm::rcp_nr); a stage whose offset is larger evaluates the point directly.  Their roundings are
+// spelled out (geodesic_accel_1).
 template <class R, bool kComp, int NS, bool kShift = false, int kUnroll = 1>
 PHX_HD void rk4_step(R a, R hs, GeoState<R, NS>& g, R dt, const StepTrig<R>& tr) {
   constexpr bool kF = NS == 12;
   static_assert(!(kShift && kComp), "the shifted stages need an uncompensated state");
   const R pi_hi = R(kPi), pi_lo = R(kPi - (double)R(kPi));
   const bool south = kComp && g.hi[2] > R(kHalfPi);
-  const R e0 = tr.e0, sx0 = tr.sx0, cx0 = tr.cx0, st0 = tr.st0, ct0 = tr.ct0;
-  const R s2x0 = R(2) * sx0 * cx0;
   R inc[NS], s03[NS], s12[NS];
 #pragma unroll
   for (int i = 0; i < NS; i++) inc[i] = R(0);
@@ -160,17 +160,17 @@ PHX_HD void rk4_step(R a, R hs, GeoState<R, NS>& g, R dt, const StepTrig<R>& tr)
     if constexpr (kShift) {
       const R d1 = inc[1], d2 = inc[2];
       if (fabs_t(d1) <= R(kShiftMax) && fabs_t(d2) <= R(kShiftMax) && fabs_t(hs) <= R(0.5)) {
+        static_assert(!kF, "the shifted stages transport no polarization vector");
         R sd, cd;
         sincos_tiny(d2, &sd, &cd);
-        const R sx = sx0 * cd + cx0 * sd, cx = cx0 * cd - sx0 * sd;
-        const R s2x = R(2) * sx * cx, c2x = (cx - sx) * (cx + sx);
+        const R sx = dprod2_1(tr.sx0, cd, tr.cx0, sd), cx = dprod2_1(tr.cx0, cd, -tr.sx0, sd);
+        const R s2x = dmul_1(2.0 * sx, cx), c2x = dmul_1(dadd_1(cx, -sx), dadd_1(cx, sx));
         // theta - theta0 = d2 + (h/2)(sin 2x2 - sin 2x2_0): |.| <= (1 + |h|) kShiftMax <= 0.0375
         R sdt, cdt;
-        sincos_tiny(d2 + R(0.5) * hs * (s2x - s2x0), &sdt, &cdt);
-        static_assert(!kF, "the shifted stages transport no polarization vector");
-        const KsPt<R> p = {e0 * exp_small<R, 7>(d1), st0 * cdt + ct0 * sdt, ct0 * cdt - st0 * sdt,
-                           R(1) + hs * c2x, R(-2) * hs * s2x};
-        geodesic_accel_ks(a, p, y + 4, d + 4);
+        sincos_tiny(dfma_1(0.5 * hs, dadd_1(s2x, -tr.s2x0()), d2), &sdt, &cdt);
+        const KsPt<R> p = {dmul_1(tr.e0, exp_small<R, 7>(d1)), dprod2_1(tr.st0, cdt, tr.ct0, sdt),
+                           dprod2_1(tr.ct0, cdt, -tr.st0, sdt), dfma_1(hs, c2x, 1.0), dmul_1(-2.0 * hs, s2x)};
+        geodesic_accel_1(a, p, y + 4, d + 4);
       } else {
         StagePoint<R> sp;
         sp.a = a;
@@ -201,7 +201,7 @@ PHX_HD void rk4_step(R a, R hs, GeoState<R, NS>& g, R dt, const StepTrig<R>& tr)
     if constexpr (kShift) {
       // one running sum d0 + 2 d1 + 2 d2 + d3 (one 8-vector of doubles fewer live through the stages)
 #pragma unroll
-      for (int i = 0; i < NS; i++) s03[i] = (q == 0 ? R(0) : s03[i]) + (q == 1 || q == 2 ? R(2) : R(1)) * d[i];
+      for (int i = 0; i < NS; i++) s03[i] = dfma_1(q == 1 || q == 2 ? 2.0 : 1.0, d[i], q == 0 ? 0.0 : s03[i]);
     } else {
 #pragma unroll
       for (int i = 0; i < NS; i++) {
@@ -214,17 +214,21 @@ PHX_HD void rk4_step(R a, R hs, GeoState<R, NS>& g, R dt, const StepTrig<R>& tr)
     if (q < 3) {
       const R wdt = (q == 2 ? R(1) : R(0.5)) * dt;
 #pragma unroll
-      for (int i = 0; i < NS; i++) inc[i] = mul_1(wdt, d[i]);
+      for (int i = 0; i < NS; i++) inc[i] = kShift ? R(dmul_1(wdt, d[i])) : mul_1(wdt, d[i]);
     }
   }
   const R dt6 = dt / R(6);
 #pragma unroll
   for (int i = 0; i < NS; i++) {
-    const R du = (kShift ? s03[i] : s03[i] + R(2) * s12[i]) * dt6;
-    if (kComp) {
-      comp_add(g.hi[i], g.lo[i], du);
+    if constexpr (kShift) {
+      g.hi[i] = dfma_1(s03[i], dt6, g.hi[i]);
     } else {
-      g.hi[i] += du;
+      const R du = (s03[i] + R(2) * s12[i]) * dt6;
+      if (kComp) {
+        comp_add(g.hi[i], g.lo[i], du);
+      } else {
+        g.hi[i] += du;
+      }
     }
   }
 }
@@ -264,15 +268,20 @@ PHX_HD R step_size(R stepsize, R x2, const R k[4], const R* dxc, R tiny, R big) 
 // The same rule with the reciprocals folded (FP32 paths): 1 / (stepsize / |k| + tiny) -> |k| / stepsize and
 // 1 / (dxc / |k| + tiny) -> |k| / dxc with the leaf's inverse cell sizes idxc, so that two divisions remain instead of
 // twelve.  Equal to step_size up to rounding; the pole term keeps the reference's 1 / tiny limit at x2 = 0.
-// kNR: the mixed mode's FP64 reciprocals (geo_rcp, geo_div).
+// kNR: the mixed mode's FP64 reciprocals (geo_rcp, geo_div), the roundings spelled out (geodesic_accel_1).
 template <class R, bool kNR = false>
 PHX_HD R step_size_fast(R stepsize, R inv_stepsize, R x2, const R k[4], const R* idxc, R tiny, R big) {
   const R a1 = fabs_t(k[1]) + tiny, a2 = fabs_t(k[2]) + tiny, a3 = fabs_t(k[3]) + tiny;
   const R m = fmin_t(x2, R(kPi) - x2);
   const R i2 = fmin_t(geo_div<R, kNR>(a2, stepsize * m), R(1) / tiny);  // m = 0: the reference's 1 / tiny
-  const R sum = (a1 + a3) * inv_stepsize + i2;
-  R grid = big;
-  if (idxc) grid = geo_div<R, kNR>(R(0.25), a1 * idxc[0] + a2 * idxc[1] + a3 * idxc[2]);
+  R sum, grid = big;
+  if constexpr (kNR) {
+    sum = dfma_1(dadd_1(a1, a3), inv_stepsize, i2);
+    if (idxc) grid = geo_div<R, kNR>(R(0.25), dfma_1(a3, idxc[2], dprod2_1(a1, idxc[0], a2, idxc[1])));
+  } else {
+    sum = (a1 + a3) * inv_stepsize + i2;
+    if (idxc) grid = geo_div<R, kNR>(R(0.25), a1 * idxc[0] + a2 * idxc[1] + a3 * idxc[2]);
+  }
   return -fmin_t(geo_rcp<R, kNR>(sum), grid);
 }
 

@@ -98,17 +98,16 @@ PHX_HD T geo_div(T a, T b) {
 
 // sin d and cos d for |d| <= 0.0375 in FP64: four Taylor terms each (truncation below 2e-17 and 1e-16 relative),
 // summed in Estrin's form (two levels of independent products instead of a three-deep Horner chain).
-template <class T>
-PHX_HD void sincos_tiny(T d, T* sn, T* cs) {
-  const T z = d * d, z2 = z * z;
-  const T s = (T(1) - z * T(1.0 / 6.0)) + z2 * (T(1.0 / 120.0) - z * T(1.0 / 5040.0));
-  const T c = (T(1) - z * T(1.0 / 2.0)) + z2 * (T(1.0 / 24.0) - z * T(1.0 / 720.0));
-  *sn = d * s;
+PHX_HD void sincos_tiny(double d, double* sn, double* cs) {
+  const double z = dmul_1(d, d), z2 = dmul_1(z, z);
+  const double s = dfma_1(z2, dfma_1(-z, 1.0 / 5040.0, 1.0 / 120.0), dfma_1(-z, 1.0 / 6.0, 1.0));
+  const double c = dfma_1(z2, dfma_1(-z, 1.0 / 720.0, 1.0 / 24.0), dfma_1(-z, 1.0 / 2.0, 1.0));
+  *sn = dmul_1(d, s);
   *cs = c;
 }
 
 // The rest of the geometry once r, sin 2x2, cos 2x2 and sin, cos of theta are known.
-template <class T, bool kNR = false>
+template <class T>
 PHX_HD KerrPt<T> kerr_point_theta(T a, T hs, T r, T s2x, T c2x, T st, T ct) {
   KerrPt<T> p;
   p.r = r;
@@ -118,13 +117,13 @@ PHX_HD KerrPt<T> kerr_point_theta(T a, T hs, T r, T s2x, T c2x, T st, T ct) {
   p.c = ct;
   p.s2 = p.s * p.s;
   p.sig = p.r * p.r + a * a * p.c * p.c;
-  p.isig = geo_rcp<T, kNR>(p.sig);  // FP32: hardware reciprocal (2 ulp), FP64: exact division or Newton-refined
+  p.isig = fastm::rcp(p.sig);  // FP32: hardware reciprocal (2 ulp), FP64: exact division
   p.q = T(2) * p.r * p.isig;
   return p;
 }
 
 // Geometry at (r, x2) when r = exp(x1) and sin x2, cos x2 are already known.
-template <class T, bool kNR = false>
+template <class T>
 PHX_HD KerrPt<T> kerr_point_rsc(T a, T hs, T r, T x2, T sx, T cx) {
   // sin 2x2, cos 2x2 from sin x2, cos x2 (double-angle identities)
   const T s2x = T(2) * sx * cx, c2x = (cx - sx) * (cx + sx);
@@ -139,7 +138,7 @@ PHX_HD KerrPt<T> kerr_point_rsc(T a, T hs, T r, T x2, T sx, T cx) {
   } else {
     sincos_t(x2 + d, &st, &ct);
   }
-  return kerr_point_theta<T, kNR>(a, hs, r, s2x, c2x, st, ct);
+  return kerr_point_theta(a, hs, r, s2x, c2x, st, ct);
 }
 
 // Geometry at (r, x2) when r = exp(x1) is already known.
@@ -169,13 +168,13 @@ PHX_HD Cov<T> cov_metric(const KerrPt<T>& p, T a) {
   return g;
 }
 
-template <class T, bool kNR = false>
+template <class T>
 PHX_HD Contra<T> contra_metric(const KerrPt<T>& p, T a) {
   Contra<T> u;
   const T isig = p.isig;
-  const T ir = geo_rcp<T, kNR>(p.r);
+  const T ir = fastm::rcp(p.r);
   const T tp2 = p.tp * p.tp;
-  const T iprod = isig * geo_rcp<T, kNR>(tp2 * p.s2);  // one reciprocal for both 1 / theta'^2 and 1 / sin^2
+  const T iprod = isig * fastm::rcp(tp2 * p.s2);  // one reciprocal for both 1 / theta'^2 and 1 / sin^2
   u.tt = -(T(1) + p.q);
   u.t1 = T(2) * isig;
   u.x11 = isig * ((p.r - T(2)) * p.r + a * a) * ir * ir;
@@ -341,7 +340,7 @@ PHX_HD void cov_derivs(const KerrPt<T>& p, T a, Cov<T>* D1, Cov<T>* D2) {
   D2->x33 = sc2 * (p.sig + a2 * p.s2 * opq) + p.s2 * (sig2 + a2 * (sc2 * opq + p.s2 * q2));
 }
 
-// What geodesic_accel_ks needs of a point: r, sin and cos of theta, theta' and theta''.
+// What geodesic_accel_1 and geodesic_accel_ks need of a point: r, sin and cos of theta, theta' and theta''.
 template <class T>
 struct KsPt {
   T r, s, c, tp, tpp;
@@ -350,11 +349,11 @@ struct KsPt {
 // Right-hand side of the geodesic equation and of the parallel transport of a polarization vector F:
 //   dk^mu/dl = -Gamma^mu_ab k^a k^b,   dF^mu/dl = -Gamma^mu_ab k^a F^b.
 // kF = false: k only (F and dF are not touched; the polarization then comes from the Walker-Penrose constant).
-template <class T, bool kF = true, bool kNR = false>
+template <class T, bool kF = true>
 PHX_HD void geodesic_accel_at(T a, const KerrPt<T>& p, const T k[4], const T F[4], T dk[4], T dF[4]) {
   Cov<T> D1, D2;
   cov_derivs(p, a, &D1, &D2);
-  const Contra<T> u = contra_metric<T, kNR>(p, a);
+  const Contra<T> u = contra_metric(p, a);
   T Pk[4], Qk[4];
   symv(D1, k, Pk);  // D1 k
   symv(D2, k, Qk);  // D2 k
@@ -386,10 +385,9 @@ PHX_HD void geodesic_accel_at(T a, const KerrPt<T>& p, const T k[4], const T F[4
 // dk^mu/dl = -Gamma^mu_ab k^a k^b from the Kerr-Schild form of the metric, g = eta + q l l with l = (1, 1, 0, -a sin^2)
 // in (t, r, theta, phi): the Euler-Lagrange equations d(g_mu nu k^nu)/dl = (d_mu g_ab) k^a k^b / 2 with the null vector's
 // contraction L = l.k taken out of every term, solved with eta's inverse (its r-phi block has determinant sin^2 Sigma)
-// and q l l, then carried from (r, theta) to (x1, x2).  About 80 operations and one reciprocal against 130 and three of
-// geodesic_accel_at, in shorter chains: the mixed march waits for FP64 results (pipe 41% active, issue 50%).  Equal to it
-// up to rounding: against 80-bit arithmetic 2.4e-16 rms of the largest component (2.0e-16), at most 1.5e-14 (1.9e-14).
-// Measured: 512^2 image, one frequency 124.6 -> 104.6 ms; 333 x 217, 3 frequencies 79.0 -> 68.5 ms.
+// and q l l, then carried from (r, theta) to (x1, x2).  No march runs it: it is a derivation of its own, which the tests hold
+// geodesic_accel_at against.  Against 80-bit arithmetic 3.3e-16 rms of the largest component of null vectors (with
+// geodesic_accel_at 2.5e-16).
 template <class T>
 PHX_HD void geodesic_accel_ks(T a, const KsPt<T>& p, const T k[4], T dk[4]) {
   const T r2 = p.r * p.r, a2 = a * a, ra = r2 + a2;
@@ -423,6 +421,67 @@ PHX_HD void geodesic_accel_ks(T a, const KsPt<T>& p, const T k[4], T dk[4]) {
   dk[1] = (dkr - kr * k[1]) * ir;
   dk[2] = (isig * ah - p.tpp * k[2] * k[2]) * itp;
   dk[3] = isig * (a * ar + ap);
+}
+
+// a b + c d, the first product inside the fused operation.
+PHX_HD double dprod2_1(double a, double b, double c, double d) { return dfma_1(a, b, dmul_1(c, d)); }
+
+PHX_HD void symv_1(const Cov<double>& m, const double V[4], double out[4]) {
+  out[0] = dfma_1(m.t3, V[3], dprod2_1(m.tt, V[0], m.t1, V[1]));
+  out[1] = dfma_1(m.x13, V[3], dprod2_1(m.t1, V[0], m.x11, V[1]));
+  out[2] = dmul_1(m.x22, V[2]);
+  out[3] = dfma_1(m.x33, V[3], dprod2_1(m.t3, V[0], m.x13, V[1]));
+}
+
+// geodesic_accel_at (k only, Newton-refined reciprocals) with every rounding spelled out: the mixed march's.  A ray of the
+// central column of an image of odd width passes the south pole at pi - x2 of 1e-11, which FP64 holds to 1e-5 only: one
+// rounding more or less, anywhere before, moves phi by 1e-5 to 1e-4 behind the pole and the image by up to 1e-2 at a pixel.
+// Left to the compiler, the contractions changed with the code around them, and those pixels with them.  The form is
+// the one that the kernels took before their frequency loop was rolled: 1 + q is fused in the x1 derivatives and
+// in g^tt and rounded twice in the x2 derivatives; of the products that two sums share, the first sum fuses the other one.
+// The Kerr-Schild form (geodesic_accel_ks) in its place is faster (512^2, one frequency 75.4 ms against 88.5; 333 x 217, 3
+// frequencies 59.5 against 69.5), but its error is a third larger, and with reciprocals of their own, which mend that, it takes 84.5.
+PHX_HD void geodesic_accel_1(double a, const KsPt<double>& p, const double k[4], double dk[4]) {
+  const double r = p.r, s = p.s, c = p.c, tp = p.tp, tpp = p.tpp;
+  const double s2 = dmul_1(s, s), a2 = dmul_1(a, a), r2 = dmul_1(r, r), tr = dmul_1(2.0, r), tr2 = dmul_1(2.0, r2);
+  const double sig = dprod2_1(r, r, dmul_1(a2, c), c), isig = fastm::rcp_nr(sig);
+  const double q = dmul_1(tr, isig), opq = dfma_1(tr, isig, 1.0), opq2 = dadd_1(q, 1.0);
+  const double as2 = dmul_1(-a, s2), a2s2 = dmul_1(a2, s2);
+  // d g / d x1 and d g / d x2 (cov_derivs)
+  const double u1 = dfma_1(-tr2, isig, 1.0), q1 = dmul_1(q, u1);
+  Cov<double> D1, D2;
+  D1.tt = q1;
+  D1.t1 = dmul_1(dfma_1(tr, isig, q1), r);
+  D1.t3 = dmul_1(as2, q1);
+  D1.x11 = dmul_1(dfma_1(2.0, opq, q1), r2);
+  D1.x13 = dmul_1(dmul_1(as2, dadd_1(q1, opq)), r);
+  D1.x22 = dmul_1(dmul_1(tr2, tp), tp);
+  D1.x33 = dmul_1(s2, dfma_1(a2s2, q1, tr2));
+  const double sc2 = dmul_1(dmul_1(dmul_1(2.0, s), c), tp), sig2 = dmul_1(-a2, sc2);
+  const double q2 = dmul_1(dmul_1(-q, sig2), isig), sq = dprod2_1(sc2, opq2, s2, q2);
+  D2.tt = q2;
+  D2.t1 = dmul_1(q2, r);
+  D2.t3 = dmul_1(-a, dprod2_1(sc2, q, s2, q2));
+  D2.x11 = dmul_1(q2, r2);
+  D2.x13 = dmul_1(dmul_1(-a, r), sq);
+  D2.x22 = dprod2_1(dmul_1(sig2, tp), tp, dmul_1(dmul_1(2.0, sig), tp), tpp);
+  D2.x33 = dprod2_1(sc2, dfma_1(a2s2, opq2, sig), s2, dfma_1(a2, sq, sig2));
+  // g^{mu nu} (contra_metric)
+  const double ir = fastm::rcp_nr(r), tp2 = dmul_1(tp, tp), iprod = dmul_1(isig, fastm::rcp_nr(dmul_1(tp2, s2)));
+  const double ut1 = dmul_1(2.0, isig), ux11 = dmul_1(dmul_1(dmul_1(isig, dprod2_1(dadd_1(r, -2.0), r, a, a)), ir), ir);
+  const double ux13 = dmul_1(dmul_1(a, isig), ir), ux22 = dmul_1(iprod, s2), ux33 = dmul_1(iprod, tp2);
+  double P[4], Q[4], f[4];
+  symv_1(D1, k, P);
+  symv_1(D2, k, Q);
+  const double kD1k = dfma_1(P[3], k[3], dfma_1(P[2], k[2], dprod2_1(P[0], k[0], P[1], k[1])));
+  const double kD2k = dfma_1(Q[3], k[3], dadd_1(dmul_1(Q[2], k[2]), dprod2_1(Q[0], k[0], Q[1], k[1])));
+  for (int n = 0; n < 4; n++) f[n] = dprod2_1(k[1], P[n], k[2], Q[n]);
+  f[1] = dfma_1(-0.5, kD1k, f[1]);
+  f[2] = dfma_1(-0.5, kD2k, f[2]);
+  dk[0] = -dprod2_1(ut1, f[1], -opq, f[0]);
+  dk[1] = -dfma_1(ux13, f[3], dprod2_1(ut1, f[0], ux11, f[1]));
+  dk[2] = -dmul_1(ux22, f[2]);
+  dk[3] = -dprod2_1(ux13, f[1], ux33, f[3]);
 }
 
 template <class T, bool kF = true>

@@ -538,7 +538,7 @@ struct Ray : GeoRay<M, PT>, PlasmaRay<M, PT, NF, typename RayStore<M, PT, NF>::A
     return Geo::template march<M == Mode::kFP32 ? kUnroll : 1>(
         sg, rc, ctr, [&](const G* x, const G* k, const G* F, G r, G hl, int right, const StepTrig<G>& tr) {
           if constexpr (Geo::kShift) {  // the step's own sines and cosines
-            const KerrPt<G> own = tr.point(sg.a, sg.hs);
+            const KerrPt<G> own = tr.point(sg.a, sg.hs, x[2]);
             Plasma::process_sample(s, sg, rc, x, k, F, r, hl, right, ctr, &own);
           } else {
             Plasma::process_sample(s, sg, rc, x, k, F, r, hl, right, ctr);
