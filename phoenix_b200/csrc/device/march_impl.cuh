@@ -1,6 +1,8 @@
 // Launch logic of the raymarch kernel (see march.cuh); each march_<mode>_nf<slots>.cu file instantiates launch_nf.
 #pragma once
 
+#include <cmath>
+
 #include "march.cuh"
 #include "march_pipe.cuh"
 
@@ -44,31 +46,45 @@ cudaError_t launch_mb(const MarchArgs<typename Policy<M>::R, PT>& args, int sms,
   return cudaGetLastError();
 }
 
-// The pipelined kernel (march_pipe.cuh) takes the launches of few rays per SM.  Its blocks hold one ray per lane of their
-// geodesic warp only, so 168 registers leave room for 192 rays an SM (128: 256) against the plain kernel's 512: it wins
-// while a launch is as long as its longest rays, and loses once the rays fill the chip several times over, the sooner the
-// longer the plasma stage is.  Plain kernel's time over the pipelined one's at 20 / 75 deg (96 x 48 x 48-base snapshot), by
-// rays per SM:
-//   FP32, 1 frequency: 28 1.6 / 1.6, 442 1.22 / 1.34, 529 1.10 / 1.17, 691 0.97 / 1.00;  2: 442 1.07 / 1.24;  3: 270 1.22 / 1.16,
-//     389 1.12 / 1.18, 492 0.91 / 0.95;  4: 492 1.09 / 1.15;  5: 389 0.94 / 0.94;  8: 172 1.58 / 1.60, 270 1.40 / 1.32;  32: 27 3.1 / 3.3, 270 2.0 / 1.8
-//   mixed, 1: 28 1.7 / 1.7, 442 1.33 / 1.52, 691 1.11 / 1.19;  2: 442 1.08 / 1.48;  3: 270 1.30 / 1.30, 492 0.90 / 0.97;  8: 67
-//     1.72 / 1.90, 270 1.16 / 1.12
-//   FP64, 1: 110 1.28 / 1.19, 297 1.21 / 1.36;  3: 67 1.26 / 1.23, 110 1.09 / 1.08, 172 0.96 / 0.98, 270 0.72 / 0.70;  8: 110 1.38 /
-//     1.53, 270 0.92 / 0.82
-// Odd widths put a column of rays over the poles that all take the most steps there are, and gain more: FP32, 351 x 333 (789)
-// 1.13 / 1.14, 3 frequencies 271 x 269 (492) 1.11 / 1.23; mixed 1.26 / 1.32 and 1.12 / 1.13.  The limits lie between the two.
-template <Mode M, int NF>
-constexpr long long pipe_rays_per_sm() {
-  return M == Mode::kFP64 ? (NF == 1 ? 300 : NF <= 4 ? 140 : 180)
-                          : NF == 1 ? (M == Mode::kFP32 ? 700 : 850) : NF <= 4 ? 500 : (M == Mode::kFP32 ? 320 : 300);
-}
-constexpr int kPipeWideRays = 490;  // rays per SM up to which a pipelined launch takes 168 registers, beyond them 128
-
 // Plasma warps of a pipelined block: one for one frequency; more frequencies make the plasma stage the longer one, so two
 // (up to 4) or four warps share them.
 template <int NF>
 constexpr int pipe_plasma_warps() {
   return NF == 1 ? 1 : NF <= 4 ? 2 : 4;
+}
+
+// Whether a line of pixels looks along the axis: the central column of an odd width (row of an odd height, turned by 90
+// degrees).  Its rays have no angular momentum, circle the poles for as many steps as there are, and make the launch as
+// long as they are.
+inline bool has_axis_line(int W, int H, double cos_pa, double sin_pa) {
+  return (W % 2 == 1 && std::fabs(sin_pa) < 1e-6) || (H % 2 == 1 && std::fabs(cos_pa) < 1e-6);
+}
+
+// The pipelined kernel (march_pipe.cuh) takes the launches of few rays per SM.  Its blocks hold one ray per lane of their
+// geodesic warp only, so 168 registers leave room for 192 rays an SM against the plain kernel's 512: it wins while a
+// launch is as long as its longest rays, and loses once the rays fill the chip several times over; the sooner the longer
+// the plasma stage is (one frequency more than the plasma warps share evenly is as long as a whole round more), and the later
+// with a line of rays along the axis.  Plain kernel's time over the pipelined one's at 20 / 75 deg (96 x 48 x 48-base snapshot, 3
+// levels), by rays per SM, even widths | odd ones:
+//   FP32, 1 frequency: 490 1.25 / 1.27, 620 1.04 / 1.17, 700 0.94 / 0.95 | 700 1.15 / 1.32, 850 1.10 / 1.13
+//     2: 490 1.15 / 1.15, 600 0.99 / 1.01 | 490 1.33 / 1.46     3: 440 1.06 / 1.09, 490 0.94 / 1.04 | 490 1.17 / 1.30
+//     4: 490 1.15 / 1.16, 540 1.03 / 1.10 | 490 1.30 / 1.51     5: 330 1.01 / 1.00 | 330 1.22 / 1.41
+//     8: 320 1.13 / 1.33 | 320 1.36 / 1.54
+//   mixed, 1: 490 1.27 / 1.37, 620 1.05 / 1.15, 700 0.96 / 0.94 | 780 1.05 / 1.14, 850 1.02 / 1.07
+//     2: 390 1.08 / 1.11, 440 1.03 / 0.95, 490 0.91 / 0.93 | 490 1.06 / 1.13, 540 1.01 / 1.14
+//     3: 330 1.11 / 1.07, 390 0.97 / 0.99, 490 0.81 / 0.86 | 440 1.06 / 1.10, 490 1.01 / 0.98 (333 x 217: 1.07 / 1.08)
+//     4: 390 1.14 / 1.19, 440 1.04 / 0.98, 490 0.97 / 0.98 | 490 1.15 / 1.14     5: 220 1.05 / 1.12, 300 0.94 / 1.03 | 300 1.25 / 1.26
+//     8: 300 1.16 / 1.32 | 300 1.41 / 1.55
+//   FP64, 1: 300 1.17 / 1.26, 340 1.02 / 1.00 | 300 1.30 / 1.35     3: 110 1.05 / 1.03, 140 1.03 / 1.23 | 140 1.14 / 1.10
+//     8: 180 1.05 / 1.35 | 180 1.27 / 1.63
+// A variant of 128 registers (256 rays an SM) was at most 4% faster, between 600 and 650 rays an SM, and slower below.
+template <Mode M, int NF>
+long long pipe_rays_per_sm(int nfreqs, bool axis_line) {
+  if (M == Mode::kFP64) return NF == 1 ? 300 : NF <= 4 ? 140 : 180;
+  const bool over = nfreqs % pipe_plasma_warps<NF>() == 1;  // NF > 1
+  if (M == Mode::kFP32) return NF == 1 ? (axis_line ? 700 : 650) : NF <= 4 ? (over && !axis_line ? 450 : 500) : 320;
+  if (axis_line) return NF == 1 ? 850 : NF <= 4 ? 500 : 300;
+  return NF == 1 ? 650 : NF <= 4 ? (over ? 360 : 420) : (over ? 240 : 300);
 }
 
 template <Mode M, class PT, int NF, int kS, int kMinCtas>
@@ -112,15 +128,11 @@ template <Mode M, class PT, int NF>
 cudaError_t launch_nf(const MarchArgs<typename Policy<M>::R, PT>& args, int sms, int blocks_per_sm,
                       cudaStream_t stream, LaunchShape* shape) {
   // a launch shape or refill policy named by the caller: always the plain kernel
-  if (blocks_per_sm <= 0 && args.default_schedule && args.njobs <= pipe_rays_per_sm<M, NF>() * sms) {
+  const bool axis_line = has_axis_line(args.rc.W, args.rc.H, args.rc.cos_pa, args.rc.sin_pa);
+  if (blocks_per_sm <= 0 && args.default_schedule &&
+      args.njobs <= pipe_rays_per_sm<M, NF>(args.rc.nfreqs, axis_line) * sms) {
     constexpr int kS = pipe_plasma_warps<NF>(), kThreads = 32 * (1 + kS);
-    if constexpr (M == Mode::kFP64) {
-      return launch_pipe<M, PT, NF, kS, 256 / kThreads>(args, sms, stream, shape);
-    } else {
-      return args.njobs <= (long long)kPipeWideRays * sms
-                 ? launch_pipe<M, PT, NF, kS, 384 / kThreads>(args, sms, stream, shape)
-                 : launch_pipe<M, PT, NF, kS, 512 / kThreads>(args, sms, stream, shape);
-    }
+    return launch_pipe<M, PT, NF, kS, (M == Mode::kFP64 ? 256 : 384) / kThreads>(args, sms, stream, shape);
   }
   if constexpr (M == Mode::kFP64) {
     (void)blocks_per_sm;
