@@ -35,7 +35,8 @@ PHX_HD void build_K(const Coeffs<R>& c, R c2, R s2, R K[4][4], R j[4]) {
 
 // E = -h P^-1 K and S = h P^-1 j by Gauss-Jordan elimination on [P | K | j], with partial pivoting (kPivot) or without:
 // while the off-diagonal entries of each column of P sum to less than its diagonal entry, pivoting exchanges nothing and
-// the two give the same bits.
+// the two give the same bits: the roundings are spelled out, as a warp takes the one or the other by what any of its lanes
+// needs, and a ray may not depend on the rays beside it.
 template <class R, bool kPivot = true>
 PHX_HD void segment_operator(const R K[4][4], const R j[4], R h, R E[4][4], R S[4]) {
   R M[4][9];
@@ -44,7 +45,7 @@ PHX_HD void segment_operator(const R K[4][4], const R j[4], R h, R E[4][4], R S[
   for (int i = 0; i < 4; i++) {
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-      M[i][k] = (i == k ? R(1) : R(0)) + hh * K[i][k];
+      M[i][k] = i == k ? fma_1(hh, K[i][k], R(1)) : mul_1(hh, K[i][k]);
       M[i][4 + k] = K[i][k];
     }
     M[i][8] = j[i];
@@ -63,20 +64,20 @@ PHX_HD void segment_operator(const R K[4][4], const R j[4], R h, R E[4][4], R S[
     }
     const R inv = fastm::rcp(M[c][c]);  // FP32: hardware reciprocal (2 ulp); FP64: exact
 #pragma unroll
-    for (int q = c; q < 9; q++) M[c][q] *= inv;
+    for (int q = c; q < 9; q++) M[c][q] = mul_1(M[c][q], inv);
 #pragma unroll
     for (int r = 0; r < 4; r++) {
       if (r == c) continue;
       const R f = M[r][c];
 #pragma unroll
-      for (int q = c; q < 9; q++) M[r][q] -= f * M[c][q];
+      for (int q = c; q < 9; q++) M[r][q] = fma_1(-f, M[c][q], M[r][q]);
     }
   }
 #pragma unroll
   for (int i = 0; i < 4; i++) {
 #pragma unroll
-    for (int k = 0; k < 4; k++) E[i][k] = -h * M[i][4 + k];
-    S[i] = h * M[i][8];
+    for (int k = 0; k < 4; k++) E[i][k] = mul_1(-h, M[i][4 + k]);
+    S[i] = mul_1(h, M[i][8]);
   }
 }
 
