@@ -232,7 +232,7 @@ void autotune(PhxBatch* b) {
   auto add = [&](int bps) {
     for (const auto& pol : policies) cand.push_back({bps, pol[0], pol[1]});
   };
-  if (b->precision == PHX_PREC_FP32 && b->nf_slots <= 4) {
+  if (b->precision == PHX_PREC_FP32) {
     for (int bps : {3, 4, 1}) add(bps);
   } else if (b->precision == PHX_PREC_MIXED && b->nf_slots == 1) {
     for (int bps : {3, 4, 1}) add(bps);
