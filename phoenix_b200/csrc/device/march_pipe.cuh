@@ -36,6 +36,7 @@ __global__ void __launch_bounds__(32 * (1 + kS), kMinCtas)
   __shared__ int32_t head_pix[32];      // the rays of this round: pixel (-1: none) and Walker-Penrose constant
   __shared__ double head_kappa[2][32];
   __shared__ int head_end;
+  __shared__ int ray_bad[32];           // bad samples of the rays of this round, over the plasma warps
   auto block_sync = [] {
     __syncwarp();
     asm volatile("bar.sync 1, %0;" ::"n"(32 * (1 + kS)) : "memory");
@@ -47,6 +48,8 @@ __global__ void __launch_bounds__(32 * (1 + kS), kMinCtas)
   if (role == 0) {
     Geo ray;
     unsigned steps = 0, rays = 0;
+    int32_t last = -1;  // the pixel of the round before
+    ray_bad[lane] = 0;
     for (;;) {
       unsigned long long base = 0;
       if (lane == 0) base = atomicAdd(&A.counters[kCtrQueue], 32ull);
@@ -68,6 +71,11 @@ __global__ void __launch_bounds__(32 * (1 + kS), kMinCtas)
       head_pix[lane] = live ? pix : -1;
       if (lane == 0) head_end = end;
       block_sync();
+      // the plasma warps are through with the round before: its counts are stored, not added up in global memory, where
+      // a pixel that is in the job list twice would get both rays'
+      if (A.pixstats && last >= 0) A.pixstats[3 * (size_t)last + 2] = ray_bad[lane];
+      ray_bad[lane] = 0;
+      last = live ? pix : -1;
       if (end) break;
       for (int b = 0;; b ^= 1) {
 #pragma unroll 1
@@ -90,11 +98,7 @@ __global__ void __launch_bounds__(32 * (1 + kS), kMinCtas)
               sampled = true;
             });
             if (!live) {
-              if (A.pixstats) {
-                int32_t* ps = A.pixstats + 3 * (size_t)ray.pix;
-                ps[0] = ray.steps;
-                ps[2] = 0;
-              }
+              if (A.pixstats) A.pixstats[3 * (size_t)ray.pix] = ray.steps;
               steps += (unsigned)ray.steps;
               rays++;
             }
@@ -146,11 +150,8 @@ __global__ void __launch_bounds__(32 * (1 + kS), kMinCtas)
       }
       if (pix >= 0) {
         ray.write(A.out, pix, A.rc.nfreqs, first);
-        if (A.pixstats) {
-          int32_t* ps = A.pixstats + 3 * (size_t)pix;
-          if (first == 0) ps[1] = ray.nplasma;
-          if (ray.bad) atomicAdd(ps + 2, ray.bad);
-        }
+        if (A.pixstats && first == 0) A.pixstats[3 * (size_t)pix + 1] = ray.nplasma;
+        if (ray.bad) atomicAdd(&ray_bad[lane], ray.bad);
         nplasma += (unsigned)ray.nplasma;
         bad += (unsigned)ray.bad;
       }
