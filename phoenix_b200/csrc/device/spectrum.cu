@@ -5,17 +5,20 @@
 //   tau, tauF   means over the pixels whose six values sum to a finite number (0 when there are none).
 //
 // One thread-block cluster per frequency: each CTA sums a strided share of the pixels into FP64 partials (warp shuffles,
-// then its warps in a fixed order); CTA 0 of the cluster then reads the other CTAs' partials through distributed shared
-// memory, in rank order, and writes the record.  The result is deterministic (no atomics) and nothing beyond the image
-// and the output records is touched.
+// then its warps in a fixed order) and writes them into CTA 0's shared memory, which adds them up in rank order and
+// writes the record.  The result is deterministic (no atomics) and nothing beyond the image and the output records is
+// touched.
 //
 // The kernel is bound by what its SMs can read, so the cluster is the largest set of SMs that can add up partials without
 // scratch memory, 16 CTAs (8, the portable size, where the device cannot place 16), and a thread loads kSpecUnroll records
-// before it adds the first.  Measured (records of three images in turn): 1024^2 pixels, 4 frequencies 178 -> 96 us, 1
-// frequency 132 -> 35 us; 512^2, 3 frequencies 42 -> 25 us; 1400 x 1300, 6 frequencies 281 -> 131 us; images up to 300^2
-// stay at the launch's 13 to 17 us.  With several frequencies every lane's record is a cache line of its own and the L1's
-// tag lookups hold an SM at 33 GB/s; three lanes to a record (shuffled verdicts: 105 us for the first of these; staged
-// through shared memory: 86, but 55 and 31 us for the next two) did not pay.
+// before it adds the first.  A CTA holds 26,624 of an SM's 65,536 registers: a spectrum starts beside another stream's
+// kernel that leaves that much free (up to three blocks of a pipelined render); with 512 threads and six records, all of an
+// SM's registers, it waited for half a render of 64^2 pixels, 3.6 ms instead of 0.03.  Measured (records of three images in
+// turn; in brackets 512 threads and six records, then 8 CTAs of 512 threads): 1024^2 pixels, 4 frequencies 95 us (93, 177), 1
+// frequency 54 (32, 134); 512^2, 3 frequencies 23.6 (23.6, 42.7); 1400 x 1300, 6 frequencies 129 (131, 277); 128^2 6.5
+// (6.6, 7.5).  With several frequencies every lane's record is a cache line of its own and the L1's tag lookups hold an SM
+// at 33 GB/s; three lanes to a record (shuffled verdicts: 105 us for the first of these; staged through shared memory:
+// 86, but 55 and 31 us for the next two) did not pay.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
@@ -33,33 +36,25 @@ using namespace phx_capi;
 namespace {
 
 constexpr int kSpecCluster = 16, kSpecClusterPortable = 8;
-constexpr int kSpecUnroll = 6;  // records a thread has in flight
-constexpr int kSpecThreads = 512;
+constexpr int kSpecUnroll = 5;  // records a thread has in flight
+constexpr int kSpecThreads = 256;
 constexpr int kSpecWarps = kSpecThreads / 32;
 
-// Sums of a warp, a CTA or the cluster.  From the warps up they are compensated: s + e is the sum, e what the additions
-// to s rounded off.  Every addition there rounds at the size of the total, and the 15 CTAs after the first alone put
-// 1e-16 on it; the threads' and the shuffles' roundings are of parts and average out.  Mean error of 24 images' totals against
-// an exact sum 9e-18 (8 CTAs without it: 6.7e-17); 2 us of 96.
-struct SpecPart {
-  double s[6], e[6];        // I, Q, U, V, tau, tauF
-  unsigned long long n[2];  // pixels in the flux sum, in the optical-depth means
-};
-
-// a += b (Knuth's two-sum; an infinite sum leaves a NaN in e, which total() drops).
-__device__ __forceinline__ void add_part(SpecPart& a, const SpecPart& b) {
-#pragma unroll
-  for (int q = 0; q < 6; q++) {
-    const double x = a.s[q], y = b.s[q], t = x + y, z = t - x;
-    a.s[q] = t;
-    a.e[q] += b.e[q] + ((x - (t - z)) + (y - z));
-  }
-  a.n[0] += b.n[0];
-  a.n[1] += b.n[1];
+// Sums of warps, CTAs and the cluster are compensated: s + e is the sum, e what the additions to s rounded off.  Every
+// addition there rounds at the size of the total, and the 15 CTAs after the first alone put 1e-16 on it; the threads' and
+// the shuffles' roundings are of parts and average out.  Of 288 totals of 512^2 images 96% are the exact sum, rounded
+// (without the compensation, 8 CTAs of 512 threads, 65%).
+//
+// (s, e) += (y, f): Knuth's two-sum, e what the additions to s rounded off (an infinite sum leaves a NaN in e, which total()
+// drops).
+__device__ __forceinline__ void add_comp(double& s, double& e, double y, double f) {
+  const double t = s + y, z = t - s;
+  e += f + ((s - (t - z)) + (y - z));
+  s = t;
 }
-__device__ __forceinline__ double total(const SpecPart& a, int q) {
-  const double t = a.s[q] + a.e[q];
-  return isfinite(t) ? t : a.s[q];
+__device__ __forceinline__ double total(double s, double e) {
+  const double t = s + e;
+  return isfinite(t) ? t : s;
 }
 
 __device__ __forceinline__ double warp_sum(double v) {
@@ -68,86 +63,93 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
-__device__ __forceinline__ unsigned long long warp_sum(unsigned long long v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  return v;
-}
-
-__global__ void __launch_bounds__(kSpecThreads)
+__global__ void __launch_bounds__(kSpecThreads, 2)
     k_spectrum(const double2* __restrict__ res, long long npix, int nfreqs, double jy_per_unit,
                PhxSpectrum* __restrict__ out) {
-  __shared__ SpecPart warp_part[kSpecWarps];
-  __shared__ SpecPart cta_part;
+  __shared__ double warp_s[6][kSpecWarps];
+  __shared__ unsigned warp_n[2][kSpecWarps];
+  __shared__ double cta_s[6][kSpecCluster], cta_e[6][kSpecCluster];  // of rank 0: every CTA's partials
+  __shared__ unsigned long long cta_n[2][kSpecCluster];
   cg::cluster_group cluster = cg::this_cluster();
+  cluster.barrier_arrive();  // waited for before the first access to rank 0's shared memory
   const unsigned rank = cluster.block_rank(), ncta = cluster.num_blocks();
   const int f = blockIdx.y;
   double s[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-  unsigned long long nflux = 0, ntau = 0;
-  const long long stride = (long long)ncta * kSpecThreads;
-  for (long long p0 = (long long)rank * kSpecThreads + threadIdx.x; p0 < npix; p0 += kSpecUnroll * stride) {
+  unsigned nflux = 0, ntau = 0;
+  const unsigned first = rank * kSpecThreads + threadIdx.x, stride = ncta * kSpecThreads;
+  int n = first < npix ? (int)(((unsigned)npix - first + stride - 1) / stride) : 0;
+  const size_t step = (size_t)stride * nfreqs * 3;
+  const double2* r = res + ((size_t)first * nfreqs + f) * 3;
+  for (; n > 0; n -= kSpecUnroll, r += kSpecUnroll * step) {
     double2 v[kSpecUnroll][3];
 #pragma unroll
     for (int u = 0; u < kSpecUnroll; u++) {
-      const long long p = p0 + u * stride;
-      if (p < npix) {
-        const double2* r = res + ((size_t)p * nfreqs + f) * 3;  // one 48-byte record: three 16-byte loads
+      if (u < n) {
 #pragma unroll
-        for (int w = 0; w < 3; w++) v[u][w] = __ldg(r + w);
+        for (int w = 0; w < 3; w++) v[u][w] = __ldg(r + u * step + w);
       }
     }
+    // the records of a round first: all but one of their additions round at their own size, not at the sum's
+    double t[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
 #pragma unroll
     for (int u = 0; u < kSpecUnroll; u++) {
-      if (p0 + u * stride >= npix) break;
+      if (u >= n) break;
       const double2 iq = v[u][0], uv = v[u][1], tt = v[u][2];
       const double stokes = iq.x + iq.y + uv.x + uv.y;
       if (isfinite(stokes)) {
-        s[0] += iq.x;
-        s[1] += iq.y;
-        s[2] += uv.x;
-        s[3] += uv.y;
+        t[0] += iq.x;
+        t[1] += iq.y;
+        t[2] += uv.x;
+        t[3] += uv.y;
         nflux++;
       }
       if (isfinite(stokes + tt.x + tt.y)) {
-        s[4] += tt.x;
-        s[5] += tt.y;
+        t[4] += tt.x;
+        t[5] += tt.y;
         ntau++;
       }
     }
+#pragma unroll
+    for (int q = 0; q < 6; q++) s[q] += t[q];
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
   for (int q = 0; q < 6; q++) s[q] = warp_sum(s[q]);
-  nflux = warp_sum(nflux);
-  ntau = warp_sum(ntau);
+  nflux = __reduce_add_sync(0xffffffffu, nflux);
+  ntau = __reduce_add_sync(0xffffffffu, ntau);
   if (lane == 0) {
 #pragma unroll
-    for (int q = 0; q < 6; q++) {
-      warp_part[warp].s[q] = s[q];
-      warp_part[warp].e[q] = 0.0;
-    }
-    warp_part[warp].n[0] = nflux;
-    warp_part[warp].n[1] = ntau;
+    for (int q = 0; q < 6; q++) warp_s[q][warp] = s[q];
+    warp_n[0][warp] = nflux;
+    warp_n[1][warp] = ntau;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    SpecPart t = warp_part[0];
-    for (int w = 1; w < kSpecWarps; w++) add_part(t, warp_part[w]);
-    cta_part = t;
+  cluster.barrier_wait();
+  const int q = threadIdx.x;
+  if (q < 6) {
+    double t = warp_s[q][0], e = 0.0;
+#pragma unroll
+    for (int w = 1; w < kSpecWarps; w++) add_comp(t, e, warp_s[q][w], 0.0);
+    *cluster.map_shared_rank(&cta_s[q][rank], 0) = t;
+    *cluster.map_shared_rank(&cta_e[q][rank], 0) = e;
+  } else if (q < 8) {
+    unsigned long long t = 0;
+    for (int w = 0; w < kSpecWarps; w++) t += warp_n[q - 6][w];
+    *cluster.map_shared_rank(&cta_n[q - 6][rank], 0) = t;
   }
-  cluster.sync();  // every CTA's partial is in its shared memory
-  if (rank == 0 && threadIdx.x == 0) {
-    SpecPart t = cta_part;
-    for (unsigned c = 1; c < ncta; c++) add_part(t, *cluster.map_shared_rank(&cta_part, c));
-    PhxSpectrum rec;
-    for (int q = 0; q < 4; q++) rec.IQUV[q] = total(t, q) * jy_per_unit;
-    rec.tau_mean = t.n[1] ? total(t, 4) / (double)t.n[1] : 0.0;
-    rec.tauF_mean = t.n[1] ? total(t, 5) / (double)t.n[1] : 0.0;
-    rec.n_flux = (int64_t)t.n[0];
-    rec.n_tau = (int64_t)t.n[1];
-    out[f] = rec;
+  cluster.sync();
+  if (rank != 0 || q >= 8) return;
+  unsigned long long m = 0;
+  for (unsigned c = 0; c < ncta; c++) m += cta_n[q == 6 ? 0 : 1][c];
+  if (q >= 6) {
+    (q == 6 ? out[f].n_flux : out[f].n_tau) = (int64_t)m;
+    return;
   }
-  cluster.sync();  // CTA 0 has read the others' shared memory before they exit
+  double t = cta_s[q][0], e = cta_e[q][0];
+  for (unsigned c = 1; c < ncta; c++) add_comp(t, e, cta_s[q][c], cta_e[q][c]);
+  t = total(t, e);
+  if (q < 4) out[f].IQUV[q] = t * jy_per_unit;
+  else (q == 4 ? out[f].tau_mean : out[f].tauF_mean) = m ? t / (double)m : 0.0;
 }
 
 // Whether the current device can place a cluster of kSpecCluster CTAs of k_spectrum (16 is beyond the portable 8).
