@@ -241,7 +241,8 @@ typedef struct {
   int32_t autotune;        /* nonzero: time every (blocks_per_sm, refill policy) candidate on a sample of the batch's
                               tiles at creation, then every tile shape at the fastest of them, and keep the fastest */
   int32_t sample_stride;   /* autotune sample: every n-th tile, 0 = 16 */
-  int32_t keep_order;      /* nonzero: tiles in item order; 0: the largest images' tiles first */
+  int32_t keep_order;      /* nonzero: tiles in item order; 0: the tiles nearest the image centres first, in bands of 2.5 M
+                              over all images, the larger images first inside a band */
   int32_t tile_shape;      /* pixel order of the items without a job list, i.e. the shape of the pixel tile a warp's
                               32 consecutive rays cover: PHX_TILE_* (0 = Morton, the reference's schedule) */
   int32_t lane_setup;      /* nonzero: each lane sets up the camera ray it takes (no start-state buffer); 0: a ray-setup

@@ -48,10 +48,6 @@ struct PhxBatch {
   unsigned long long* ctl = nullptr;
   unsigned long long* counters = nullptr;
   int tile_rays = 32;
-  std::vector<phx::TileDesc> image_tiles;  // the tiles image by image, before place_tiles orders them
-  std::vector<int32_t> host_jobs;          // the job lists on the device, for place_tiles
-  bool keep_order = false;
-  int sample_stride = 16;
   phx::QueueShape shape{3, 32};
   phx::LaunchShape lshape{};
   PhxBatchTuning tuning{};
@@ -97,31 +93,39 @@ std::vector<int32_t> pixel_order(int32_t W, int32_t H, int shape) {
   return m;
 }
 
+// What the tiles are ordered from, while the batch is created.
+struct TileOrder {
+  std::vector<phx::TileDesc> image_tiles;  // the tiles image by image
+  std::vector<int32_t> jobs;               // the job lists on the device
+  bool keep_order;
+  int sample_stride;
+};
+
 // Orders the tiles for the current job lists and uploads them, and every sample_stride-th for the trials.  Long rays first:
 // they pass within about 8 M of the hole, so unless the caller keeps its order the tiles nearest the image centres go
 // first over all images, in bands of kBand, the images together inside a band.  Image by image, the launch ended with the
 // last images' longest rays: 24 images of 48 to 256 pixels a side 87.2 -> 79.7 ms, 32 mixed 208 -> 192, 128 images of up to 512
 // pixels 1923 -> 1904 (two bands of 8 M: 83.4, 196.9, 1894).
-void place_tiles(PhxBatch* b) {
+void place_tiles(PhxBatch* b, const TileOrder& o) {
   constexpr double kBand = 2.5;
   constexpr int kBands = 8;
-  std::vector<phx::TileDesc> tiles = b->image_tiles;
-  if (!b->keep_order) {
+  std::vector<phx::TileDesc> tiles = o.image_tiles;
+  if (!o.keep_order) {
     std::vector<std::pair<int, int32_t>> by(tiles.size());  // band, tile
     for (size_t t = 0; t < tiles.size(); t++) {
       const PhxRenderParams& p = b->params[tiles[t].item];
-      const int32_t pix = b->host_jobs[b->job_off[tiles[t].item] + tiles[t].first + tiles[t].count / 2];
+      const int32_t pix = o.jobs[b->job_off[tiles[t].item] + tiles[t].first + tiles[t].count / 2];
       const double x = (pix / p.img_height + 0.5) / p.img_width - 0.5;
       const double y = (pix % p.img_height + 0.5) / p.img_height - 0.5;
       const double d = std::hypot(x * p.fov_x, y * p.fov_y) / kBand;
       by[t] = {d < kBands - 1 ? (int)d : kBands - 1, (int32_t)t};
     }
     std::sort(by.begin(), by.end());
-    for (size_t t = 0; t < tiles.size(); t++) tiles[t] = b->image_tiles[by[t].second];
+    for (size_t t = 0; t < tiles.size(); t++) tiles[t] = o.image_tiles[by[t].second];
   }
   std::vector<phx::TileDesc> trial;
   b->trial_rays = 0;
-  for (size_t t = 0; t < tiles.size(); t += b->sample_stride) {
+  for (size_t t = 0; t < tiles.size(); t += o.sample_stride) {
     trial.push_back(tiles[t]);
     b->trial_rays += tiles[t].count;
   }
@@ -131,15 +135,15 @@ void place_tiles(PhxBatch* b) {
 }
 
 // Writes every own-order item's job list for `shape` into the device job array.
-void upload_order(PhxBatch* b, int shape) {
+void upload_order(PhxBatch* b, TileOrder& o, int shape) {
   for (size_t i = 0; i < b->params.size(); i++) {
     if (!b->own_order[i]) continue;
     const std::vector<int32_t> m = pixel_order(b->params[i].img_width, b->params[i].img_height, shape);
     ck(cudaMemcpy(b->jobs + b->job_off[i], m.data(), m.size() * sizeof(int32_t), cudaMemcpyHostToDevice), "H2D jobs");
-    std::copy(m.begin(), m.end(), b->host_jobs.begin() + b->job_off[i]);
+    std::copy(m.begin(), m.end(), o.jobs.begin() + b->job_off[i]);
   }
   b->tile_shape = shape;
-  place_tiles(b);
+  place_tiles(b, o);
 }
 
 unsigned pow2_mask(int64_t n) {
@@ -225,7 +229,7 @@ void run_setup(PhxBatch* b) {
   ck(cudaStreamSynchronize(b->stream), "ray setup");
 }
 
-void autotune(PhxBatch* b) {
+void autotune(PhxBatch* b, TileOrder& order) {
   std::vector<phx::QueueShape> cand;
   // refill policies: the finished lanes every 128 passes; a warp with 24 finished lanes; a warp with all 32 finished
   const int policies[3][2] = {{128, 1}, {phx::kDefaultQueuePeriod, 24}, {phx::kDefaultQueuePeriod, 32}};
@@ -271,7 +275,7 @@ void autotune(PhxBatch* b) {
   if (any_own) {
     for (int shape = 0; shape < PHX_TILE_SHAPES; shape++) {
       if (shape == shape0) continue;
-      upload_order(b, shape);
+      upload_order(b, order, shape);
       run_setup(b);
       const float ms = timed_launch(b, b->trial, b->ntrial, b->trial_mask, b->trial_rays, b->shape, &ls);
       record(b->shape, shape, ms);
@@ -280,7 +284,7 @@ void autotune(PhxBatch* b) {
         best_shape = shape;
       }
     }
-    if (b->tile_shape != best_shape) upload_order(b, best_shape);
+    if (b->tile_shape != best_shape) upload_order(b, order, best_shape);
   }
   b->tuning.ncand = nc;
 }
@@ -376,8 +380,6 @@ PhxBatch* create_batch(const PhxBatchItem* items, int32_t nitems, const PhxBatch
   b->ntiles = (int64_t)tiles.size();
   b->nrays = std::accumulate(b->njobs.begin(), b->njobs.end(), (int64_t)0);
   b->ntrial = (b->ntiles + o.sample_stride - 1) / o.sample_stride;
-  b->sample_stride = o.sample_stride;
-  b->keep_order = o.keep_order != 0;
   b->tile_mask = pow2_mask(std::max<int64_t>(b->ntiles, 1));
   b->trial_mask = pow2_mask(std::max<int64_t>(b->ntrial, 1));
   // device buffers
@@ -392,9 +394,8 @@ PhxBatch* create_batch(const PhxBatchItem* items, int32_t nitems, const PhxBatch
   b->counters = b->alloc<unsigned long long>(phx::kNumCounters);
   b->tiles = b->alloc<phx::TileDesc>((size_t)b->tile_mask + 1);
   b->trial = b->alloc<phx::TileDesc>((size_t)b->trial_mask + 1);
-  b->image_tiles = std::move(tiles);
-  b->host_jobs = std::move(all_jobs);
-  place_tiles(b.get());
+  TileOrder placed{std::move(tiles), std::move(all_jobs), o.keep_order != 0, o.sample_stride};
+  place_tiles(b.get(), placed);
   switch (b->precision) {
     case PHX_PREC_FP32:
       build_items<phx::Mode::kFP32, float>(b.get(), items, nitems, job_off);
@@ -417,7 +418,7 @@ PhxBatch* create_batch(const PhxBatchItem* items, int32_t nitems, const PhxBatch
                   : (b->precision == PHX_PREC_FP32 ? 4 : b->precision == PHX_PREC_MIXED ? (b->nf_slots == 1 ? 4 : 3) : 1),
               o.period > 0 ? o.period : phx::kDefaultQueuePeriod, o.refill_lanes > 0 ? o.refill_lanes : 32};
   run_setup(b.get());
-  if (o.autotune && b->ntrial > 0) autotune(b.get());
+  if (o.autotune && b->ntrial > 0) autotune(b.get(), placed);
   capture(b.get());
   b->tuning.blocks_per_sm = b->shape.blocks_per_sm;
   b->tuning.period = b->shape.period;
