@@ -198,8 +198,8 @@ PHX_HD void cell_weights(const SnapView<R, PT>& s, int leaf, const R x[4], int c
 #pragma unroll
   for (int d = 0; d < 3; d++) {
     const R lb = ldg(s.lb + 3 * leaf + d), dx = ldg(s.dxc + 3 * leaf + d);
-    // FP32 and kRcp: one reciprocal per axis instead of two divisions (rounding-level difference; the interpolant is
-    // continuous across cells)
+    // FP32 and kRcp: one reciprocal per axis instead of two divisions (rounding-level difference in u, and the interpolant is
+    // continuous across cells; kRcp: the weight is the rounded quotient all the same)
     constexpr bool kByRcp = sizeof(R) == 4 || kRcp;
     const R idx = kByRcp ? geo_rcp<R, kRcp>(dx) : R(0);
     const R u = kByRcp ? mul_1(x[1 + d] - lb, idx) : (x[1 + d] - lb) / dx;
@@ -208,7 +208,7 @@ PHX_HD void cell_weights(const SnapView<R, PT>& s, int leaf, const R x[4], int c
     if (c[d] < 0) c[d] = 0;  // unreachable for finite points of the leaf; keeps every gather inside the block
     const int ix = kFloorBy1000 ? (int)(u + R(1000)) - 1000 : (int)floor_t(u);
     const R off = x[1 + d] - fma_1(R(ix), dx, lb);
-    del[d] = (ix < 0) ? R(0) : (ix > s.nx[d] - 2) ? R(1) : (kByRcp ? mul_1(off, idx) : off / dx);
+    del[d] = (ix < 0) ? R(0) : (ix > s.nx[d] - 2) ? R(1) : (kByRcp ? geo_quot<R, kRcp>(off, dx, idx) : off / dx);
   }
 }
 

@@ -83,3 +83,45 @@ def test_no_further_from_extended_precision(tmp_path):
     assert v[6] <= 5e-14, v
     for at, one in ((v[0], v[1]), (v[2], v[3]), (v[4], v[5])):
         assert one <= 1.01 * at, v
+
+
+QUOT_SRC = r"""
+#include <cmath>
+#include <cstdio>
+#include <cstdint>
+#include "kerr.cuh"
+using namespace phx;
+
+int main() {
+  uint64_t s = 0x9E3779B97F4A7C15ull;
+  auto u01 = [&]() { s ^= s << 13; s ^= s >> 7; s ^= s << 17; return (double)(s >> 11) / 9007199254740992.0; };
+  int off = 0, far = 0, plain = 0;
+  for (int i = 0; i < 4000000; i++) {
+    // offsets in a block over its cell size
+    const double dx = std::exp(-12 + 12 * u01()), a = (i % 16 ? u01() * 64 : 1e-6 * u01()) * dx;
+    const double ib = geo_rcp<double, true>(dx), q = geo_quot<double, true>(a, dx, ib), e = a / dx;
+    off += q != e;
+    far += std::fabs(q - e) > std::nextafter(std::fabs(e), 1e308) - std::fabs(e);
+    plain += a * ib != e;
+  }
+  // an exact multiple of the cell size stays one
+  int whole = 0;
+  for (int n = 0; n < 4096; n++) {
+    const double dx = std::ldexp(1.0, -n % 40);
+    whole += geo_quot<double, true>(n * dx, dx, geo_rcp<double, true>(dx)) != n;
+  }
+  std::printf("%d %d %d %d\n", off, far, whole, plain);
+  return 0;
+}
+"""
+
+
+def test_cell_weights_quotient(tmp_path):
+    """The quotient from a reciprocal within an ulp is off by at most one ulp, and only where a/b lies next to the middle of
+    two numbers: the remainder's correction errs by about 2^-53 ulp x 2^52, so one in some thousands."""
+    src, exe = tmp_path / "q.cpp", tmp_path / "q"
+    src.write_text(QUOT_SRC)
+    core = os.path.join(ROOT, "phoenix_b200", "csrc", "core")
+    subprocess.check_call(["g++", "-O2", "-std=c++17", "-ffp-contract=off", "-I" + core, str(src), "-o", str(exe)])
+    off, far, whole, plain = map(int, subprocess.check_output([str(exe)]).decode().split())
+    assert far == 0 and whole == 0 and off <= 4000 and plain > 400000, (off, far, whole, plain)
