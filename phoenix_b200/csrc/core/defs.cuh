@@ -92,9 +92,9 @@ PHX_HD T fmod_t(T x, T y) {
 }
 
 // a b and a b + c with the rounding spelled out in FP32 device code: mul_1 is never contracted into an addition, fma_1
-// always rounds once.  The plasma stage uses them where its result decides something (emission cuts), so that every
-// kernel built from it (register cap, frequency slots, queue) decides alike; left to the compiler, the choice changed
-// with the code around it and moved about 7 of 3e8 samples across a cut.  FP64 and host code keep plain arithmetic.
+// always rounds once.  The plasma stage uses them where its result decides something (emission cuts): left to the compiler,
+// the choice changed with the code around it and moved about 7 of 3e8 samples across a cut.  FP32 kernels all decide alike;
+// mixed ones have three forms (PlasmaRay::kSig).  FP64 and host code keep plain arithmetic.
 #if defined(__CUDA_ARCH__)
 PHX_D float mul_1(float a, float b) { return __fmul_rn(a, b); }
 PHX_D float fma_1(float a, float b, float c) { return __fmaf_rn(a, b, c); }

@@ -452,7 +452,7 @@ PHX_HD void symv_1(const Cov<double>& m, const double V[4], double out[4]) {
 // the one that the kernels took before their frequency loop was rolled: 1 + q is fused in the x1 derivatives and
 // in g^tt and rounded twice in the x2 derivatives; of the products that two sums share, the first sum fuses the other one.
 // The Kerr-Schild form (geodesic_accel_ks) in its place is faster (512^2, one frequency 75.4 ms against 88.5; 333 x 217, 3
-// frequencies 59.5 against 69.5), but its error is a third larger, and with reciprocals of their own, which mend that, it takes 84.5.
+// frequencies 59.5 against 69.5), but its error is a third larger; with reciprocals of their own, which mend that, it takes 84.5.
 PHX_HD void geodesic_accel_1(double a, const KsPt<double>& p, const double k[4], double dk[4]) {
   const double r = p.r, s = p.s, c = p.c, tp = p.tp, tpp = p.tpp;
   const double s2 = dmul_1(s, s), a2 = dmul_1(a, a), r2 = dmul_1(r, r), tr = dmul_1(2.0, r), tr2 = dmul_1(2.0, r2);

@@ -294,10 +294,12 @@ struct PlasmaRay : RayTypes<M, PT> {
   using R = typename T::R;
   using G = typename T::G;
   using T::kComp, T::kMixed, T::kWP;
-  // Which way the sample's Sigma and B^2 (kSig: sample_point, derive_fluid) and g^tt (kGtt: sample_metric) are rounded: the
-  // mixed kernels of one slot (not the queue's) have always had another form of the first two than the rest, those of up to
-  // 4 slots (the queue's: of one) of the last, and a sample on an emission cut or next to a field line turns on the last
-  // bit.
+  // Which way the sample's Sigma and B^2 (kSig: sample_point, derive_fluid) and g^tt (kGtt: sample_metric) are rounded.  FP32
+  // kernels have one form.  The mixed kernels' images were made with three, which differ in the last bit: in one slot
+  // (not the queue's) the first two, in up to 4 slots (the queue's: in one) the last.  They stay, as a sample on an emission
+  // cut turns on that bit: a mixed image of one frequency, of several, and of a batch may decide such a sample (some in 10^8)
+  // otherwise.  The pitch angle's cut below is left to the compiler; no kernel has shown another choice of it than the plain one
+  // of its slots (sample counts of 40 images, pixel by pixel).
   static constexpr bool kSig = !(kMixed && NF == 1 && !kQueue);
   static constexpr bool kGtt = !(kMixed && NF <= (kQueue ? 1 : 4));
 

@@ -42,3 +42,26 @@ def test_column_over_the_poles(gpu_snapshots, incl, nfreqs, kernel):
     n = min(nfreqs, 3)
     got = res[W // 2, :, :n, 4:]
     assert (np.abs(got - ref[:, :n]).max(axis=0) <= 5e-7 * np.abs(ref[:, :n]).max(axis=0)).all()
+
+
+@pytest.mark.parametrize("incl", [20.0, 75.0])
+def test_pipelined_and_plain_sample_alike(gpu_snapshots, incl):
+    """An image of odd width and three frequencies, 488 rays an SM: the same samples in every pixel, Faraday depths to 1e-5
+    of the largest (the bound of separately compiled coefficients, far below what one sample more or less moves)."""
+    import torch
+    snap, W, H = gpu_snapshots["cfg1"], 333, 217
+    jobs = torch.from_numpy(P.schedule_morton(W, H)).cuda()
+    out = []
+    for refill in (0, 24):
+        p = P.make_params(img_width=W, img_height=H, inclination=incl, phi=33.0, m_unit=1e19, precision="mixed",
+                          frequencies=[86e9, 172e9, 344e9])
+        p.refill_lanes = refill
+        res = torch.zeros(W * H, 3, 6, dtype=torch.float64, device="cuda")
+        ps = torch.zeros(W * H, 3, dtype=torch.int32, device="cuda")
+        ctr = torch.zeros(P.NUM_COUNTERS, dtype=torch.int64, device="cuda")
+        snap.render_async(p, jobs.data_ptr(), W * H, res.data_ptr(), ctr.data_ptr(), ps.data_ptr(),
+                          stream=torch.cuda.current_stream().cuda_stream)
+        out.append((res.cpu().numpy(), ps.cpu().numpy()))
+    (a, pa), (b, pb) = out
+    assert np.array_equal(pa, pb)
+    assert (np.abs(a[..., 5] - b[..., 5]).max(axis=0) <= 1e-5 * np.abs(b[..., 5]).max(axis=0)).all()
